@@ -21,6 +21,7 @@
 #include "gemm_epilogue.cuh"
 #include "gemm_tc.h"
 #include "kernels.h"
+#include "umma.cuh"
 
 #include <stdlib.h>
 
@@ -32,105 +33,198 @@ namespace nfai {
 
 namespace {
 
+using namespace umma;
+
 constexpr int kBM = 128;
 constexpr int kBK = 64;  // halves per stage row = 128 bytes = one swizzle span
 constexpr int kGemmThreads = 192;
-constexpr unsigned long long kGemmWaitNs = 1000000000ull;
+constexpr uint32_t kEpiWarp = 32 * 32 * 4;  // an epilogue warp's shared memory
 
-__device__ __forceinline__ unsigned long long g_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ uint32_t s_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// ---- epilogue of an accumulator tile ------------------------------------------------------------------------------
+// tcgen05.ld hands every lane one accumulator row; the output wants lanes along a row. A 32 x 32 block goes through 4 KB of
+// shared memory in 16-byte quads (quad j of row r lies at place j ^ (r & 7): neither side conflicts) and comes back with 8 lanes
+// on the 32 columns of a row, 4 rows per instruction, all of it in registers before the first store: 8 wide loads and stores per
+// lane and block. Stores of single columns or pairs from the accumulator's layout touched 32 rows per instruction: 256 x 2048 at
+// K = 64 took 8.0 us, now 3.6; 128 x 16384 x 2048 (67 MB of weights) 34 us.
 
-__device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+// Whether every quad of columns that lies below N can be read and written in one piece
+template <int KIND>
+__device__ __forceinline__ bool quads_fit(const GemmEpilogue& ep, uint32_t N) {
+  auto aligned = [](const void* p, uint32_t bytes) { return ((uintptr_t)p & (bytes - 1)) == 0; };
+  if (N & 3u) return false;
+  const uint32_t act_bytes = ep.out_dtype == 0 ? 4 : 2;
+  if constexpr (KIND == GEMM_EPI_STORE) return aligned(ep.out_f32, 16) && aligned(ep.resid, 16) && aligned(ep.bias, 16);
+  if constexpr (KIND == GEMM_EPI_GATED) return aligned(ep.out_act, 2 * act_bytes) && aligned(ep.bias, 16);
+  if constexpr (KIND == GEMM_EPI_GATED_CLAMPED) return (ep.gated_cols & 3u) == 0 && aligned(ep.out_act, 2 * act_bytes) && aligned(ep.out_f32, 16);
+  if constexpr (KIND == GEMM_EPI_STORE_ACT) return aligned(ep.out_act, 4 * act_bytes) && aligned(ep.bias, 16);
+  const uint32_t row = ep.kv_f16 ? 8 : 16;
+  return ((ep.qDim | ep.kvDim | ep.d | ep.ropeDim) & 3u) == 0 && aligned(ep.out_f32, 16) && aligned(ep.kcache, row) && aligned(ep.vcache, row) &&
+         aligned(ep.rope_cs, 16);
 }
-__device__ __forceinline__ void bar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+// two consecutive activations at element `at`, in their type
+__device__ __forceinline__ void store_acts2(const GemmEpilogue& ep, size_t at, float a, float b) {
+  if (ep.out_dtype == 1) *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(ep.out_act) + at) = __floats2half2_rn(a, b);
+  else if (ep.out_dtype == 2) *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(ep.out_act) + at) = __floats2bfloat162_rn(a, b);
+  else *reinterpret_cast<float2*>(reinterpret_cast<float*>(ep.out_act) + at) = make_float2(a, b);
 }
-__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
+__device__ __forceinline__ uint2 half_quad(const float4& v) {
+  const __half2 a = __floats2half2_rn(v.x, v.y), b = __floats2half2_rn(v.z, v.w);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
-// Bounded wait; false after one second.
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
-  if (bar_try(bar, parity)) return true;
-  const unsigned long long t0 = g_ns();
-  uint32_t polls = 0;
-  while (!bar_try(bar, parity)) {
-    if ((++polls & 63u) == 0 && g_ns() - t0 > kGemmWaitNs) return false;
+__device__ __forceinline__ uint2 bf16_quad(const float4& v) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+
+// One warp's share of a tile: columns from `acc` of tensor memory, rows [m0, M) of the output, the quarter lane_grp of the
+// lanes, column blocks c_first, c_first + c_step, ... of `blocks`, 32 columns each, from n0; eb is its 4 KB of shared memory.
+// What the epilogue reads besides the sums (residual, (cos, sin) pairs) is fetched a block ahead, first before the wait for the
+// accumulator.
+template <int KIND>
+__device__ __forceinline__ bool tile_epilogue(const GemmEpilogue& ep, const uint32_t m0, const uint32_t M, const uint32_t n0, const uint32_t N,
+                                              const int blocks, const uint32_t acc, const uint32_t lane_grp, const int c_first, const int c_step,
+                                              const int lane, const uint32_t eb, const uint32_t tfull, const uint32_t parity) {
+  constexpr bool kRope = KIND == GEMM_EPI_QKV_ROPE, kRows = KIND == GEMM_EPI_STORE || kRope;  // kRows: reads something per row
+  const uint32_t quad = lane & 7, mrow = m0 + lane_grp * 32 + (lane >> 3);                     // rows mrow, mrow + 4, ... of the block
+  const bool fit = quads_fit<KIND>(ep, N);
+  float4 aux[8];
+  // everything about a quad of Q/K/V that depends on the column only: which of Q, K, V; its place there; whether it is rotated
+  struct Place {
+    uint32_t seg, local, e;
+    bool rot;
+  };
+  auto place = [&](uint32_t n) {
+    Place c;
+    c.seg = n < ep.qDim ? 0u : n < ep.qDim + ep.kvDim ? 1u : 2u;
+    c.local = n - (c.seg == 0 ? 0u : c.seg == 1 ? ep.qDim : ep.qDim + ep.kvDim);
+    c.e = c.local & (ep.d - 1);  // head dimensions are powers of two (32, 64, 128)
+    c.rot = c.seg < 2 && c.e < ep.ropeDim;
+    return c;
+  };
+  auto load_aux = [&](int b) {
+    const uint32_t n = n0 + b * 32 + quad * 4;
+    if constexpr (kRope) {
+      const Place c = place(n);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        aux[i] = c.rot && n < N && mrow + 4 * i < M
+                     ? __ldg(reinterpret_cast<const float4*>(ep.rope_cs + (size_t)(ep.pos0 + mrow + 4 * i) * (ep.ropeDim / 2) + (c.e >> 1)))
+                     : make_float4(1.f, 0.f, 1.f, 0.f);
+    } else {
+      const float4 bias = ep.bias && n < N ? __ldg(reinterpret_cast<const float4*>(ep.bias + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ep.resid && n < N && mrow + 4 * i < M) r = __ldcg(reinterpret_cast<const float4*>(ep.resid + (size_t)(mrow + 4 * i) * N + n));
+        aux[i] = make_float4(r.x + bias.x, r.y + bias.y, r.z + bias.z, r.w + bias.w);
+      }
+    }
+  };
+  if (kRows && fit) load_aux(c_first);
+  bool good = bar_wait(tfull, parity);
+  good = __all_sync(0xffffffffu, good);
+  if (!good) return false;
+  fence_after();
+#pragma unroll 1
+  for (int b = c_first; b < blocks; b += c_step) {
+    const uint32_t nb = n0 + b * 32, n = nb + quad * 4;
+    float4 x[8];
+    {
+      uint32_t v[32];
+      tmem_ld(acc + ((lane_grp * 32u) << 16) + (uint32_t)b * 32u, v);
+      if (m0 + lane_grp * 32 >= M || nb >= N) continue;  // (warp-uniform)
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(eb + lane * 128 + ((j ^ (lane & 7)) << 4)), "r"(v[4 * j]), "r"(v[4 * j + 1]),
+                     "r"(v[4 * j + 2]), "r"(v[4 * j + 3])
+                     : "memory");
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t r = (lane >> 3) + 4 * i;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(x[i].x), "=f"(x[i].y), "=f"(x[i].z), "=f"(x[i].w)
+                     : "r"(eb + r * 128 + ((quad ^ (r & 7)) << 4))
+                     : "memory");
+      }
+      __syncwarp();
+    }
+    if (!fit) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t m = mrow + 4 * i;
+        if (m >= M || n >= N) continue;
+        epilogue_pair<KIND>(ep, m, n, N, x[i].x, x[i].y, epilogue_aux<KIND>(ep, m, n, N));
+        if (n + 2 < N) epilogue_pair<KIND>(ep, m, n + 2, N, x[i].z, x[i].w, epilogue_aux<KIND>(ep, m, n + 2, N));
+      }
+      continue;
+    }
+    if constexpr (KIND == GEMM_EPI_STORE) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = make_float4(aux[i].x + x[i].x, aux[i].y + x[i].y, aux[i].z + x[i].z, aux[i].w + x[i].w);
+    } else if constexpr (kRope) {
+      if (n < N && place(n).rot) {  // value1 = cos*a - sin*b ; value2 = sin*a + cos*b, products rounded separately
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float4 cs = aux[i], v = x[i];
+          x[i].x = __fsub_rn(__fmul_rn(cs.x, v.x), __fmul_rn(cs.y, v.y));
+          x[i].y = __fadd_rn(__fmul_rn(cs.y, v.x), __fmul_rn(cs.x, v.y));
+          x[i].z = __fsub_rn(__fmul_rn(cs.z, v.z), __fmul_rn(cs.w, v.w));
+          x[i].w = __fadd_rn(__fmul_rn(cs.w, v.z), __fmul_rn(cs.z, v.w));
+        }
+      }
+    }
+    if constexpr (kRows) {
+      if (b + c_step < blocks) load_aux(b + c_step);  // in flight during this block's stores
+    }
+    if (n >= N) continue;
+    const int rows = mrow < M ? min(8u, (M - mrow + 3) / 4) : 0;  // of this lane's eight
+    if constexpr (KIND == GEMM_EPI_STORE) {
+      float* const out = ep.out_f32 + (size_t)mrow * N + n;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < rows) *reinterpret_cast<float4*>(out + (size_t)(4 * i) * N) = x[i];
+    } else if constexpr (kRope) {
+      const Place c = place(n);
+      const size_t kv = (size_t)(ep.pos0 + mrow) * ep.kvDim + c.local;
+      void* const cache = c.seg == 1 ? ep.kcache : ep.vcache;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (i >= rows) continue;
+        if (c.seg == 0) *reinterpret_cast<float4*>(ep.out_f32 + (size_t)(mrow + 4 * i) * ep.qDim + c.local) = x[i];
+        else if (ep.kv_f16) *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(cache) + kv + (size_t)(4 * i) * ep.kvDim) = half_quad(x[i]);
+        else *reinterpret_cast<float4*>(reinterpret_cast<float*>(cache) + kv + (size_t)(4 * i) * ep.kvDim) = x[i];
+      }
+    } else if constexpr (KIND == GEMM_EPI_GATED) {  // columns (2j, 2j+1) = (gate_j, up_j)
+      const float4 bias = ep.bias ? __ldg(reinterpret_cast<const float4*>(ep.bias + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < rows)
+          store_acts2(ep, (size_t)(mrow + 4 * i) * (N / 2) + (n >> 1), gated(ep.act, x[i].x + bias.x, x[i].y + bias.y),
+                      gated(ep.act, x[i].z + bias.z, x[i].w + bias.w));
+    } else if constexpr (KIND == GEMM_EPI_GATED_CLAMPED) {
+      const uint32_t cols = ep.gated_cols ? ep.gated_cols : N;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (i >= rows) continue;
+        if (n < cols)
+          store_acts2(ep, (size_t)(mrow + 4 * i) * (cols / 2) + (n >> 1), gated_clamped(x[i].x, x[i].y, ep.act_limit),
+                      gated_clamped(x[i].z, x[i].w, ep.act_limit));
+        else *reinterpret_cast<float4*>(ep.out_f32 + (size_t)(mrow + 4 * i) * (N - cols) + (n - cols)) = x[i];
+      }
+    } else {  // plain store in the operand type of the next product
+      const float4 bias = ep.bias ? __ldg(reinterpret_cast<const float4*>(ep.bias + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (i >= rows) continue;
+        const float4 v = make_float4(x[i].x + bias.x, x[i].y + bias.y, x[i].z + bias.z, x[i].w + bias.w);
+        const size_t at = (size_t)(mrow + 4 * i) * N + n;
+        if (ep.out_dtype == 0) *reinterpret_cast<float4*>(reinterpret_cast<float*>(ep.out_act) + at) = v;
+        else *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(ep.out_act) + at) = ep.out_dtype == 1 ? half_quad(v) : bf16_quad(v);
+      }
+    }
   }
   return true;
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(map), "r"(c0), "r"(c1), "r"(bar)
-      : "memory");
-}
-
-// Shared-memory matrix descriptor: K-major tile, 128-byte swizzle, rows of 128 bytes, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFF) >> 4);   // start address, 16-byte units
-  d |= (uint64_t)1 << 16;                     // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;           // stride byte offset: next 8-row group
-  d |= (uint64_t)1 << 46;                     // descriptor version (sm_100)
-  d |= (uint64_t)2 << 61;                     // layout: 128-byte swizzle
-  return d;
-}
-
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,"
-      "%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// 32 consecutive output columns [n0, n0+32) of row m (n0 is a multiple of 32)
-__device__ __forceinline__ void epilogue_cols(const GemmEpilogue& ep, uint32_t m, uint32_t n0, uint32_t N, const float (&v)[32]) {
-  float2 aux[16];
-#pragma unroll
-  for (int i = 0; i < 32; i += 2) aux[i >> 1] = n0 + i < N ? epilogue_aux(ep, m, n0 + i, N) : make_float2(0.f, 0.f);
-#pragma unroll
-  for (int i = 0; i < 32; i += 2)
-    if (n0 + i < N) epilogue_pair(ep, m, n0 + i, N, v[i], v[i + 1], aux[i >> 1]);
-}
-
-// Split-K: raw partial sums of the same 32 columns into [split][M][N]
-__device__ __forceinline__ void partial_cols(float* part, uint32_t m, uint32_t n0, uint32_t N, const float (&v)[32]) {
-  float* out = part + (size_t)m * N + n0;
-#pragma unroll
-  for (int i = 0; i < 32; ++i)
-    if (n0 + i < N) out[i] = v[i];
 }
 
 // Second kernel of a split GEMM: one thread per column pair adds the partials in split order and applies the epilogue.
@@ -158,10 +252,12 @@ struct GemmSmem {
   static constexpr uint32_t kBBytes = BN * kBK * 2;
   static constexpr uint32_t kStage = kABytes + kBBytes;
   static constexpr uint32_t kBarOff = STAGES * kStage;
-  static constexpr uint32_t kTotal = kBarOff + 256 + 1024;  // barriers + slack for the 1024-byte alignment
+  static constexpr uint32_t kEpiOff = kBarOff + 256;
+  static constexpr uint32_t kTotal = kEpiOff + 4 * kEpiWarp + 1024;  // slack for the 1024-byte alignment
 };
 
-template <int BN, int STAGES>
+// (KIND: the epilogue; a split stores raw partial sums into [split][M][N], the finishing kernel applies it)
+template <int BN, int STAGES, int KIND>
 __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA,
                                                                const __grid_constant__ CUtensorMap mapW, uint32_t M,
                                                                uint32_t N, uint32_t K, const GemmEpilogue ep,
@@ -235,20 +331,13 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_cons
   } else {
     // epilogue warps 2..5: warp w may touch tensor-memory lanes 32*(w%4) .. +31
     const uint32_t lane_grp = (uint32_t)(warp & 3);
-    ok = bar_wait(accbar, 0);
-    ok = __all_sync(0xffffffffu, ok);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok) {
-      const uint32_t m = m0 + lane_grp * 32 + lane;
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        float v[32];
-        tmem_ld32(tmem_base + ((lane_grp * 32u) << 16) + (uint32_t)c * 32u, v);
-        if (m < M && n0 + c * 32 < N) {
-          if (gridDim.z > 1) partial_cols(ep.scratch + (size_t)blockIdx.z * M * N, m, n0 + c * 32, N, v);
-          else epilogue_cols(ep, m, n0 + c * 32, N, v);
-        }
-      }
+    const uint32_t eb = s_u32(gsm + SM::kEpiOff) + (warp - 2) * kEpiWarp;
+    if (gridDim.z > 1) {
+      GemmEpilogue part;
+      part.out_f32 = ep.scratch + (size_t)blockIdx.z * M * N;
+      ok = tile_epilogue<GEMM_EPI_STORE>(part, m0, M, n0, N, BN / 32, tmem_base, lane_grp, 0, 1, lane, eb, accbar, 0);
+    } else {
+      ok = tile_epilogue<KIND>(ep, m0, M, n0, N, BN / 32, tmem_base, lane_grp, 0, 1, lane, eb, accbar, 0);
     }
   }
   if (!ok) {
@@ -265,12 +354,9 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_cons
   }
 }
 
-// ---- persistent variant: 128 x 256 tiles, two accumulators in tensor memory ------------------------------------
-// A 128 x 128 tile needs 32 KB of operands per 262 tensor-pipe cycles (125 B/clk per SM, about what L2 delivers), so
-// the kernel above is fed at half speed; a 128 x 256 tile needs 48 KB per 524 cycles. One CTA per SM walks tiles
-// blockIdx.x, + gridDim.x, ... (token tiles fastest, so that CTAs running together share one weight tile); the
-// accumulator alternates between two 256-column halves of tensor memory, so the epilogue of tile i (tcgen05.ld,
-// fused epilogue, global stores) runs while the tensor pipe is already on tile i + 1.
+// ---- rows in groups: 128 x 256 tiles, two accumulators in tensor memory -------------------------------------------
+// One CTA per SM walks tiles blockIdx.x, + gridDim.x, ...; the accumulator alternates between two 256-column halves of tensor
+// memory, so the epilogue of tile i (tcgen05.ld, fused epilogue, global stores) runs while the tensor pipe is on tile i + 1.
 constexpr int kPBN = 256;
 constexpr int kPStages = 4;
 struct PSmem {
@@ -278,27 +364,22 @@ struct PSmem {
   static constexpr uint32_t kBBytes = kPBN * kBK * 2;
   static constexpr uint32_t kStage = kABytes + kBBytes;
   static constexpr uint32_t kBarOff = kPStages * kStage;
-  static constexpr uint32_t kEpiOff = kBarOff + 256;             // 8 warps x 32 x 33 floats: accumulator block turned
-  static constexpr uint32_t kEpiBytes = 8 * 32 * 33 * 4;         // so that lanes run along a row of the output
+  static constexpr uint32_t kEpiOff = kBarOff + 256;
+  static constexpr uint32_t kEpiBytes = 8 * kEpiWarp;
   static constexpr uint32_t kTotal = kEpiOff + kEpiBytes + 1024;
 };
-
-__device__ __forceinline__ void bar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 
 // Eight epilogue warps, two per quarter of the tensor-memory lanes (a warp may only read the lanes of its index modulo 4),
 // each pair sharing the column blocks of its rows: with one warp per scheduler the SiLU epilogue (an exponential and
 // an IEEE division per output) ran at the latency of its dependent instructions and took longer than the tile's MMAs.
 constexpr int kPThreadsGemm = 64 + 8 * 32;
-static_assert(PSmem::kTotal <= 227 * 1024, "shared memory of the persistent kernel");
-// GROUPED: the tiles of rows come from a device list, each with the group whose matrix it is multiplied by; a tile may read
-// rows of A or W beyond its group (they exist or are zero-filled), its epilogue stores the group's own.
-template <bool GROUPED>
-__global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap mapA,
-                                                                          const __grid_constant__ CUtensorMap mapW, const uint32_t M_all,
-                                                                          uint32_t N, uint32_t K, const GemmGroups grp, const GemmEpilogue ep,
-                                                                          uint32_t* err) {
+static_assert(PSmem::kTotal <= 227 * 1024, "shared memory of the grouped kernel");
+// The tiles of rows come from a device list, each with the group whose matrix it is multiplied by; a tile may read rows of A or
+// W beyond its group (they exist or are zero-filled), its epilogue stores the group's own.
+template <int KIND>
+__global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapW,
+                                                                       uint32_t N, uint32_t K, const GemmGroups grp, const GemmEpilogue ep,
+                                                                       uint32_t* err) {
   using SM = PSmem;
   constexpr int STAGES = kPStages;
   extern __shared__ unsigned char gsm_raw[];
@@ -310,7 +391,6 @@ __global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_persistent_kernel(const
                  tempty0 = s_u32(bars + 2 * STAGES + 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t KT = (K + kBK - 1) / kBK;
-  uint32_t mtiles = (M_all + kBM - 1) / kBM;
   const uint32_t ntiles = (N + kPBN - 1) / kPBN;
 
   if (threadIdx.x == 0) {
@@ -336,24 +416,18 @@ __global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_persistent_kernel(const
   // barriers and tensor memory are set up; the operands (and the residual) come from the previous kernel
   pdl_launch_dependents();
   pdl_wait();
-  if constexpr (GROUPED) mtiles = min(*grp.n_tiles, grp.max_tiles);
-  const uint32_t tiles = mtiles * ntiles;
+  const uint32_t tiles = min(*grp.n_tiles, grp.max_tiles) * ntiles;
   struct Tile {
     uint32_t m0, m_end, n0, w0;  // rows [m0, m_end) of A and the output, columns from n0, rows of W from w0
   };
   auto tile_at = [&](uint32_t tile) {
     Tile t;
-    if constexpr (GROUPED) {  // column tiles fastest: they share the rows of A, which few other tiles do
-      const uint2 g = __ldcg(grp.tiles + tile / ntiles);
-      t.m0 = g.y;
-      t.m_end = __ldcg(grp.rows + g.x + 1);
-      t.n0 = (tile % ntiles) * kPBN;
-      t.w0 = g.x * N + t.n0;
-    } else {
-      t.m0 = (tile % mtiles) * kBM;
-      t.m_end = M_all;
-      t.n0 = t.w0 = (tile / mtiles) * kPBN;
-    }
+    // column tiles fastest: they share the rows of A, which few other tiles do
+    const uint2 g = __ldcg(grp.tiles + tile / ntiles);
+    t.m0 = g.y;
+    t.m_end = __ldcg(grp.rows + g.x + 1);
+    t.n0 = (tile % ntiles) * kPBN;
+    t.w0 = g.x * N + t.n0;
     return t;
   };
 
@@ -405,134 +479,8 @@ __global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_persistent_kernel(const
     for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++i) {
       const uint32_t acc = i & 1;
       const Tile at = tile_at(tile);
-      const uint32_t m0 = at.m0, n0 = at.n0, M = at.m_end;
-      // this lane's 16 pairs of a 32 x 32 block: lanes 0-15 along the column pairs of one row, lanes 16-31 on the next
-      const uint32_t col = 2u * (lane & 15);
-      float* eb = reinterpret_cast<float*>(gsm + SM::kEpiOff) + (warp - 2) * (32 * 33);
-      // One instance per epilogue kind, chosen once per tile: the loops below are straight-line code for that kind.
-      auto tile_epilogue = [&](auto kind_c) -> bool {
-        constexpr int KIND = decltype(kind_c)::value;
-        // residual pairs / (cos, sin) pairs come from memory per row; a bias pair is the same for all rows of a lane's block
-        constexpr bool kAux = KIND == GEMM_EPI_STORE || KIND == GEMM_EPI_QKV_ROPE;
-        float2 aux[16];
-        // Q/K/V columns: everything that depends on the column only (which of Q, K, V; the position inside the head;
-        // whether the pair is rotated) is the same for the 16 pairs of a lane in one block and is worked out once.
-        struct ColInfo {
-          uint32_t seg, local, half_e;  // 0 = Q, 1 = K, 2 = V; column inside the segment; index into a (cos, sin) row
-          bool rot, live;
-        };
-        auto col_info = [&](int c) {
-          ColInfo ci;
-          const uint32_t n = n0 + c * 32 + col;
-          ci.live = n < N;
-          ci.seg = n < ep.qDim ? 0u : n < ep.qDim + ep.kvDim ? 1u : 2u;
-          ci.local = n - (ci.seg == 0 ? 0u : ci.seg == 1 ? ep.qDim : ep.qDim + ep.kvDim);
-          const uint32_t e = ci.local & (ep.d - 1);  // head dimensions are powers of two (32, 64, 128)
-          ci.rot = ci.seg < 2 && e < ep.ropeDim;
-          ci.half_e = e >> 1;
-          return ci;
-        };
-        auto load_aux = [&](int c) {
-          if constexpr (KIND == GEMM_EPI_QKV_ROPE) {
-            const ColInfo ci = col_info(c);
-            const float2* cs = ep.rope_cs + (size_t)(ep.pos0 + m0 + lane_grp * 32 + (lane >> 4)) * (ep.ropeDim / 2) + ci.half_e;
-#pragma unroll
-            for (int rr = 0; rr < 16; ++rr) {
-              const uint32_t m = m0 + lane_grp * 32 + 2u * rr + (lane >> 4);
-              aux[rr] = ci.rot && ci.live && m < M ? cs[(size_t)(2 * rr) * (ep.ropeDim / 2)] : make_float2(1.f, 0.f);
-            }
-          } else if constexpr (kAux) {
-#pragma unroll
-            for (int rr = 0; rr < 16; ++rr) {
-              const uint32_t m = m0 + lane_grp * 32 + 2u * rr + (lane >> 4), n = n0 + c * 32 + col;
-              aux[rr] = m < M && n < N ? epilogue_aux<KIND>(ep, m, n, N) : make_float2(0.f, 0.f);
-            }
-          }
-        };
-        const int c_first = (warp - 2) >> 2;  // this warp's column blocks: c_first, c_first + 2, ...
-        load_aux(c_first);  // on its way while the tensor pipe still works on this tile
-        bool good = bar_wait(tfull0 + 8 * acc, (i >> 1) & 1);
-        good = __all_sync(0xffffffffu, good);
-        if (!good) return false;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // tcgen05.ld hands every lane one accumulator row; stores along a row would touch 32 different rows per
-        // instruction. The 32 x 32 block goes through shared memory (row stride 33: conflict-free both ways) and comes
-        // back with lanes 0-15 on the column pairs of one row and lanes 16-31 on the next row: 128-byte coalesced rows.
-#pragma unroll 1
-        for (int c = c_first; c < kPBN / 32; c += 2) {
-          float v[32];
-          tmem_ld32(tmem_base + ((lane_grp * 32u) << 16) + acc * (uint32_t)kPBN + (uint32_t)c * 32u, v);
-          const bool live = m0 + lane_grp * 32 < M && n0 + c * 32 < N;  // warp-uniform
-          if (live) {
-#pragma unroll
-            for (int e = 0; e < 32; ++e) eb[lane * 33 + e] = v[e];
-            __syncwarp();
-          }
-          float2 cur[16];
-          float2 col_bias = make_float2(0.f, 0.f);
-          if constexpr (!kAux) {
-            const uint32_t n = n0 + c * 32 + col;
-            if (n < N) col_bias = epilogue_aux<KIND>(ep, 0, n, N);
-          }
-          if constexpr (kAux) {
-#pragma unroll
-            for (int rr = 0; rr < 16; ++rr) cur[rr] = aux[rr];
-            if (c + 2 < kPBN / 32) load_aux(c + 2);  // the next block's reads are in flight during this block's stores
-          }
-          if constexpr (KIND == GEMM_EPI_QKV_ROPE) {
-            if (live) {
-              const ColInfo ci = col_info(c);
-              const uint32_t mrow = m0 + lane_grp * 32 + (lane >> 4);  // rows mrow, mrow + 2, ...
-              if (ci.live) {
-                // destination of row mrow; the next pair of this lane lies two rows (positions) further on
-                float* qd = ep.out_f32 + (size_t)mrow * ep.qDim + ci.local;
-                const size_t kvoff = (size_t)(ep.pos0 + mrow) * ep.kvDim + ci.local;
-                void* const cache = ci.seg == 1 ? ep.kcache : ep.vcache;
-#pragma unroll
-                for (int rr = 0; rr < 16; ++rr) {
-                  const uint32_t row = 2u * rr + (lane >> 4);
-                  if (mrow + 2u * rr >= M) break;
-                  float a = eb[row * 33 + col], b = eb[row * 33 + col + 1];
-                  if (ci.rot) {  // value1 = cos*a - sin*b ; value2 = sin*a + cos*b, products rounded separately
-                    const float2 cs = cur[rr];
-                    const float v1 = __fsub_rn(__fmul_rn(cs.x, a), __fmul_rn(cs.y, b));
-                    const float v2 = __fadd_rn(__fmul_rn(cs.y, a), __fmul_rn(cs.x, b));
-                    a = v1;
-                    b = v2;
-                  }
-                  if (ci.seg == 0) {
-                    *reinterpret_cast<float2*>(qd + (size_t)(2 * rr) * ep.qDim) = make_float2(a, b);
-                  } else if (ep.kv_f16) {
-                    *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(cache) + kvoff + (size_t)(2 * rr) * ep.kvDim) =
-                        __floats2half2_rn(a, b);
-                  } else {
-                    *reinterpret_cast<float2*>(reinterpret_cast<float*>(cache) + kvoff + (size_t)(2 * rr) * ep.kvDim) =
-                        make_float2(a, b);
-                  }
-                }
-              }
-              __syncwarp();
-            }
-          } else if (live) {
-#pragma unroll
-            for (int rr = 0; rr < 16; ++rr) {
-              const uint32_t row = 2u * rr + (lane >> 4);
-              const uint32_t m = m0 + lane_grp * 32 + row, n = n0 + c * 32 + col;
-              if (m < M && n < N)
-                epilogue_pair<KIND>(ep, m, n, N, eb[row * 33 + col], eb[row * 33 + col + 1], kAux ? cur[rr] : col_bias);
-            }
-            __syncwarp();
-          }
-        }
-        return true;
-      };
-      switch (ep.kind) {
-        case GEMM_EPI_STORE: ok = tile_epilogue(std::integral_constant<int, (int)GEMM_EPI_STORE>{}); break;
-        case GEMM_EPI_GATED_CLAMPED: ok = tile_epilogue(std::integral_constant<int, (int)GEMM_EPI_GATED_CLAMPED>{}); break;
-        case GEMM_EPI_GATED: ok = tile_epilogue(std::integral_constant<int, (int)GEMM_EPI_GATED>{}); break;
-        case GEMM_EPI_STORE_ACT: ok = tile_epilogue(std::integral_constant<int, (int)GEMM_EPI_STORE_ACT>{}); break;
-        default: ok = tile_epilogue(std::integral_constant<int, (int)GEMM_EPI_QKV_ROPE>{}); break;
-      }
+      ok = tile_epilogue<KIND>(ep, at.m0, at.m_end, at.n0, N, kPBN / 32, tmem_base + acc * (uint32_t)kPBN, lane_grp, (warp - 2) >> 2, 2, lane,
+                               s_u32(gsm + SM::kEpiOff) + (warp - 2) * kEpiWarp, tfull0 + 8 * acc, (i >> 1) & 1);
       if (!ok) break;
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -551,6 +499,135 @@ __global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_persistent_kernel(const
   if (warp == 1) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
   }
+}
+
+// ---- two SMs per tile: 256 x BN, each CTA of a pair holds 128 rows of A, half of the rows of W and 128 rows of the result ----
+// A 128 x 256 tile per SM reads 48 KB of operands per 512 cycles of the tensor pipe; here it is 32 KB (BN = 256), so the copies
+// keep up with the products, and narrower tiles (BN = 160: 83 bytes per cycle, below the 96 of the former) do so too: BN is
+// chosen per shape so that the last wave of pairs is as full as possible (pair_columns). One CTA pair per two SMs walks tiles,
+// token tiles fastest, so that pairs running together share one weight tile; two accumulators of 256 columns, so the epilogue of
+// a tile runs beside the products of the next.
+// Each CTA's warp 0 copies its own operands and counts them on the first CTA's barrier; the first CTA's warp 1 issues the
+// products of both; epilogues by eight warps of each CTA, its rows. Measured against a 128 x 256 tile per SM (us, 1.9 GHz):
+// 2011 x 16384 x 2048 112 against 120, 2011 x 3072 x 8192 94 and 103, 9472 x 16384 x 2048 496 and 528, 1024 x 28672 x 4096 192
+// and 208, 2011 x 2048 x 2048 22.6 and 21.8.
+constexpr int kPairStages = 6;
+struct PairSmem {
+  static constexpr uint32_t kABytes = kBM * kBK * 2;
+  static constexpr uint32_t kStage = kABytes + 128 * kBK * 2;
+  static constexpr uint32_t kBarOff = kPairStages * kStage;
+  static constexpr uint32_t kEpiOff = kBarOff + 256;
+  static constexpr uint32_t kTotal = kEpiOff + PSmem::kEpiBytes + 1024;
+};
+static_assert(PairSmem::kTotal <= 227 * 1024, "shared memory of the pair kernel");
+
+template <int KIND>
+__global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap mapA,
+                                                                    const __grid_constant__ CUtensorMap mapW, const uint32_t M, const uint32_t N,
+                                                                    const uint32_t K, const uint32_t BN, const GemmEpilogue ep, uint32_t* err) {
+  using SM = PairSmem;
+  constexpr int STAGES = kPairStages;
+  extern __shared__ unsigned char gsm_raw[];
+  unsigned char* gsm = reinterpret_cast<unsigned char*>(((uintptr_t)gsm_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(gsm + SM::kBarOff);
+  // as in the grouped kernel; "full" and "accumulator empty" count in the first CTA, the others in both
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+  const uint32_t full0 = s_u32(bars), empty0 = s_u32(bars + STAGES), tfull0 = s_u32(bars + 2 * STAGES), tempty0 = s_u32(bars + 2 * STAGES + 2);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank(), KT = (K + kBK - 1) / kBK;
+  const uint32_t mtiles = (M + 2 * kBM - 1) / (2 * kBM), tiles = mtiles * ((N + BN - 1) / BN);
+  const uint32_t first = blockIdx.x >> 1, step = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      bar_init(full0 + 8 * s, 1);
+      bar_init(empty0 + 8 * s, 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      bar_init(tfull0 + 8 * a, 1);
+      bar_init(tempty0 + 8 * a, 16);  // the epilogue warps of both CTAs
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_u32(tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  fence_before();
+  __syncthreads();
+  cluster_sync();  // the other CTA's barriers are there
+  fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  bool ok = true;
+  pdl_launch_dependents();
+  pdl_wait();
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const uint32_t b_bytes = BN / 2 * kBK * 2;
+      uint32_t it = 0;
+      for (uint32_t tile = first; tile < tiles && ok; tile += step) {
+        const uint32_t m0 = (tile % mtiles) * (2 * kBM) + rank * kBM, w0 = (tile / mtiles) * BN + rank * (BN / 2);
+        for (uint32_t kt = 0; kt < KT; ++kt, ++it) {
+          const uint32_t s = it % STAGES;
+          if (it >= (uint32_t)STAGES) {
+            if (!bar_wait(empty0 + 8 * s, ((it / STAGES) - 1) & 1)) { ok = false; break; }
+          }
+          const uint32_t a_dst = s_u32(gsm + s * SM::kStage), b_dst = a_dst + SM::kABytes, full = in_leader(full0 + 8 * s);
+          if (rank == 0) bar_expect_tx(full0 + 8 * s, 2 * (SM::kABytes + b_bytes));
+          tma_load_2d_pair(a_dst, &mapA, (int)(kt * kBK), (int)m0, full);
+          tma_load_2d_pair(b_dst, &mapW, (int)(kt * kBK), (int)w0, full);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {
+      const uint32_t idesc = (1u << 4) | (ep.operands_bf16 << 7) | (ep.operands_bf16 << 10) | ((BN >> 3) << 17) | ((uint32_t)(2 * kBM >> 4) << 24);
+      uint32_t it = 0, i = 0;
+      for (uint32_t tile = first; tile < tiles && ok; tile += step, ++i) {
+        const uint32_t acc = i & 1;
+        if (i >= 2) {  // both epilogues must have drained this half of tensor memory
+          if (!bar_wait_cluster(tempty0 + 8 * acc, ((i >> 1) - 1) & 1)) { ok = false; break; }
+          fence_after();
+        }
+        const uint32_t d = tmem_base + acc * 256u;
+        for (uint32_t kt = 0; kt < KT; ++kt, ++it) {
+          const uint32_t s = it % STAGES;
+          if (!bar_wait_cluster(full0 + 8 * s, (it / STAGES) & 1)) { ok = false; break; }
+          fence_after();
+          const uint32_t a_s = s_u32(gsm + s * SM::kStage), b_s = a_s + SM::kABytes;
+#pragma unroll
+          for (int k = 0; k < kBK / 16; ++k)
+            umma_f16_pair(d, smem_desc_sw128(a_s + k * 32), smem_desc_sw128(b_s + k * 32), idesc, (kt | (uint32_t)k) != 0);
+          umma_commit_pair(empty0 + 8 * s);
+        }
+        if (ok) umma_commit_pair(tfull0 + 8 * acc);
+      }
+    }
+  } else {
+    const uint32_t lane_grp = (uint32_t)(warp & 3);
+    uint32_t i = 0;
+    for (uint32_t tile = first; tile < tiles; tile += step, ++i) {
+      const uint32_t acc = i & 1, m0 = (tile % mtiles) * (2 * kBM) + rank * kBM, n0 = (tile / mtiles) * BN;
+      ok = tile_epilogue<KIND>(ep, m0, M, n0, N, (int)(BN / 32), tmem_base + acc * 256u, lane_grp, (warp - 2) >> 2, 2, lane,
+                               s_u32(gsm + SM::kEpiOff) + (warp - 2) * kEpiWarp, tfull0 + 8 * acc, (i >> 1) & 1);
+      if (!ok) break;
+      fence_before();
+      __syncwarp();
+      if (lane == 0) bar_arrive_cluster(in_leader(tempty0 + 8 * acc));
+    }
+  }
+  if (!ok) {
+    if (lane == 0 && err) atomicOr(err, 4u);
+    // copies and products of the pair may still be in flight: a bounded time for them to end before their memory is released
+    for (volatile uint32_t spin = 0; spin < (1u << 20); ++spin) {
+    }
+  }
+  fence_before();
+  __syncthreads();
+  cluster_sync();  // nobody arrives on, or multiplies from, the memory of a CTA that has left
+  fence_after();
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
 }
 
 // ---- small producers of the float16 A operands ----------------------------------------------------------------
@@ -601,7 +678,6 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// [rows][K] float16, K contiguous; box = 64 halves x box_rows rows, 128-byte swizzle, zero fill outside.
 // A descriptor depends only on (address, rows, K, box rows); a prompt re-uses the same few hundred of them for every
 // chunk, so they are kept per host thread instead of being encoded again at each of ~130 launches per chunk.
 struct MapKey {
@@ -616,7 +692,9 @@ struct MapKeyHash {
   }
 };
 
-bool make_map(CUtensorMap* map, const __half* base, uint64_t rows, uint64_t K, uint32_t box_rows) {
+}  // namespace
+
+bool tile_map16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32_t box_rows) {
   static thread_local std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
   const MapKey key{base, rows, K, box_rows};
   auto it = cache.find(key);
@@ -630,7 +708,7 @@ bool make_map(CUtensorMap* map, const __half* base, uint64_t rows, uint64_t K, u
   cuuint64_t strides[1] = {K * 2};
   cuuint32_t box[2] = {(cuuint32_t)kBK, box_rows};
   cuuint32_t estr[2] = {1, 1};
-  if (fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  if (fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return false;
   if (cache.size() > 4096) cache.clear();
@@ -638,12 +716,14 @@ bool make_map(CUtensorMap* map, const __half* base, uint64_t rows, uint64_t K, u
   return true;
 }
 
-template <int BN, int STAGES>
-cudaError_t launch_bn(cudaStream_t s, const __half* A, const __half* W, uint32_t M, uint32_t N, uint32_t K,
-                      const GemmEpilogue& ep, uint32_t* err, uint32_t Z = 1) {
+namespace {
+
+template <int BN, int STAGES, int KIND>
+cudaError_t launch_bn_kind(cudaStream_t s, const __half* A, const __half* W, uint32_t M, uint32_t N, uint32_t K,
+                      const GemmEpilogue& ep, uint32_t* err, uint32_t Z) {
   CUtensorMap mapA, mapW;
-  if (!make_map(&mapA, A, M, K, kBM) || !make_map(&mapW, W, N, K, BN)) return cudaErrorInvalidValue;
-  auto kern = gemm_tc_kernel<BN, STAGES>;
+  if (!tile_map16(&mapA, A, M, K, kBM) || !tile_map16(&mapW, W, N, K, BN)) return cudaErrorInvalidValue;
+  auto kern = gemm_tc_kernel<BN, STAGES, KIND>;
   const size_t smem = GemmSmem<BN, STAGES>::kTotal;
   static thread_local int attr_device = -1;  // the attribute is per device: set it once per (thread, device)
   int dev = 0;
@@ -663,12 +743,30 @@ cudaError_t launch_bn(cudaStream_t s, const __half* A, const __half* W, uint32_t
                     (const float*)ep.scratch, M, N, Z, ep);
 }
 
-template <bool GROUPED>
-cudaError_t launch_persistent(cudaStream_t s, const __half* A, const __half* W, uint32_t M, uint32_t N, uint32_t K,
-                              const GemmGroups& grp, const GemmEpilogue& ep, uint32_t* err) {
+// f(kind) with the epilogue kind as a constant
+template <typename F>
+cudaError_t with_kind(int kind, F f) {
+  switch (kind) {
+    case GEMM_EPI_STORE: return f(std::integral_constant<int, GEMM_EPI_STORE>{});
+    case GEMM_EPI_GATED: return f(std::integral_constant<int, GEMM_EPI_GATED>{});
+    case GEMM_EPI_GATED_CLAMPED: return f(std::integral_constant<int, GEMM_EPI_GATED_CLAMPED>{});
+    case GEMM_EPI_STORE_ACT: return f(std::integral_constant<int, GEMM_EPI_STORE_ACT>{});
+    default: return f(std::integral_constant<int, GEMM_EPI_QKV_ROPE>{});
+  }
+}
+
+template <int BN, int STAGES>
+cudaError_t launch_bn(cudaStream_t s, const __half* A, const __half* W, uint32_t M, uint32_t N, uint32_t K, const GemmEpilogue& ep, uint32_t* err,
+                      uint32_t Z = 1) {
+  return with_kind(ep.kind, [&](auto kind) { return launch_bn_kind<BN, STAGES, decltype(kind)::value>(s, A, W, M, N, K, ep, err, Z); });
+}
+
+template <int KIND>
+cudaError_t launch_grouped(cudaStream_t s, const __half* A, const __half* W, uint32_t max_rows, uint32_t N, uint32_t K, const GemmGroups& grp,
+                           const GemmEpilogue& ep, uint32_t* err) {
   CUtensorMap mapA, mapW;
-  if (!make_map(&mapA, A, M, K, kBM) || !make_map(&mapW, W, GROUPED ? (uint64_t)grp.count * N : N, K, kPBN)) return cudaErrorInvalidValue;
-  auto kern = gemm_tc_persistent_kernel<GROUPED>;
+  if (!tile_map16(&mapA, A, max_rows, K, kBM) || !tile_map16(&mapW, W, (uint64_t)grp.count * N, K, kPBN)) return cudaErrorInvalidValue;
+  auto kern = gemm_tc_grouped_kernel<KIND>;
   static thread_local int attr_device = -1;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -678,9 +776,43 @@ cudaError_t launch_persistent(cudaStream_t s, const __half* A, const __half* W, 
     if (e != cudaSuccess) return e;
     attr_device = dev;
   }
-  const uint32_t tiles = (GROUPED ? grp.max_tiles : (M + kBM - 1) / kBM) * ((N + kPBN - 1) / kPBN);
-  return launch_pdl(kern, dim3(tiles < sm_count() ? tiles : sm_count()), dim3(kPThreadsGemm), PSmem::kTotal, s, prefill_pdl(), mapA, mapW,
-                    M, N, K, grp, ep, err);
+  const uint32_t tiles = grp.max_tiles * ((N + kPBN - 1) / kPBN);
+  return launch_pdl(kern, dim3(tiles < sm_count() ? tiles : sm_count()), dim3(kPThreadsGemm), PSmem::kTotal, s, prefill_pdl(), mapA, mapW, N, K,
+                    grp, ep, err);
+}
+
+// Columns of a pair's tile: the width in steps of 32 that needs the least time in waves of pairs (a wave costs its width, and
+// about 8 columns' worth of filling and draining), the wider one of two equal ones. 2011 x 3072 x 8192, forced: 256: 94.1 us,
+// 192 (the choice): 94.9, 160: 129, 128: 128; 2011 x 3072 x 2048: 34.6, 32.0, 41.3, 40.4; 2011 x 16384 x 2048: 116 at 256 (the
+// choice), 123 at 224, 132 at 192.
+uint32_t pair_columns(uint32_t M, uint32_t N) {
+  const uint32_t pairs = sm_count() / 2, mt = (M + 2 * kBM - 1) / (2 * kBM);
+  uint32_t best = 256, cost = ~0u;
+  for (uint32_t bn = 256; bn >= 128; bn -= 32) {
+    const uint32_t tiles = mt * ((N + bn - 1) / bn), c = (tiles + pairs - 1) / pairs * (bn + 8);
+    if (c < cost) best = bn, cost = c;
+  }
+  return best;
+}
+
+template <int KIND>
+cudaError_t launch_pair(cudaStream_t s, const __half* A, const __half* W, uint32_t M, uint32_t N, uint32_t K, const GemmEpilogue& ep, uint32_t* err) {
+  const uint32_t BN = pair_columns(M, N);
+  CUtensorMap mapA, mapW;
+  if (!tile_map16(&mapA, A, M, K, kBM) || !tile_map16(&mapW, W, N, K, BN / 2)) return cudaErrorInvalidValue;
+  auto kern = gemm_tc_pair_kernel<KIND>;
+  static thread_local int attr_device = -1;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (attr_device != dev) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PairSmem::kTotal);
+    if (e != cudaSuccess) return e;
+    attr_device = dev;
+  }
+  const uint32_t tiles = (M + 2 * kBM - 1) / (2 * kBM) * ((N + BN - 1) / BN), pairs = sm_count() / 2;
+  return launch_pdl_cluster(kern, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kPThreadsGemm), 2, PairSmem::kTotal, s, prefill_pdl(), mapA, mapW,
+                            M, N, K, BN, ep, err);
 }
 
 }  // namespace
@@ -704,9 +836,9 @@ cudaError_t launch_gemm_tc(cudaStream_t s, const __half* A, const __half* W, uin
   if (ep.operands_bf16 > 1) return cudaErrorInvalidValue;
   // enough CTAs to pull weights with every SM when the chunk is a single row of tiles
   const uint32_t mtiles = (M + kBM - 1) / kBM;
-  // enough 128 x 256 tiles to occupy most SMs: the persistent kernel (NFAI_GEMM_PERSISTENT=0 keeps the tile-per-CTA one)
-  static const bool persistent_ok = [] { const char* v = getenv("NFAI_GEMM_PERSISTENT"); return !(v && atoi(v) == 0); }();
-  if (persistent_ok && mtiles * ((N + 255) / 256) >= 96) return launch_persistent<false>(s, A, W, M, N, K, GemmGroups(), ep, err);
+  // enough tiles to occupy most pairs of SMs
+  if (mtiles * ((N + 255) / 256) >= 96)
+    return with_kind(ep.kind, [&](auto kind) { return launch_pair<decltype(kind)::value>(s, A, W, M, N, K, ep, err); });
   if (ep.scratch) {
     uint32_t Z = gemm_tc_splits(M, N, K);
     while (Z > 1 && (size_t)Z * M * N > ep.scratch_floats) --Z;
@@ -722,7 +854,10 @@ cudaError_t launch_gemm_tc_grouped(cudaStream_t s, const __half* A, const __half
   static_assert(kGroupTile == kBM, "the tile list is made for this kernel's tiles");
   if (!A || !W || !max_rows || !N || !K || (K & 7u) || (((uintptr_t)A | (uintptr_t)W) & 15) || !g.count || !g.max_tiles) return cudaErrorInvalidValue;
   if (ep.kind == GEMM_EPI_QKV_ROPE || ((ep.kind == GEMM_EPI_GATED || ep.kind == GEMM_EPI_GATED_CLAMPED) && (N & 1u)) || ep.bias || ep.resid || ep.operands_bf16 > 1) return cudaErrorInvalidValue;
-  return launch_persistent<true>(s, A, W, max_rows, N, K, g, ep, err);
+  return with_kind(ep.kind, [&](auto kind) {
+    if constexpr (decltype(kind)::value == GEMM_EPI_QKV_ROPE) return cudaErrorInvalidValue;
+    else return launch_grouped<decltype(kind)::value>(s, A, W, max_rows, N, K, g, ep, err);
+  });
 }
 
 bool prefill_pdl() {
