@@ -269,6 +269,9 @@ cudaError_t launch_attn_prefill(cudaStream_t s, int kvdtype, const AttnParams& p
 // The same contract on the tensor cores (d = 64 or 128): a CTA owns 64 tokens of one head and walks the prefix once.
 bool attn_prefill_tc_supported(uint32_t d);
 cudaError_t launch_attn_prefill_tc(cudaStream_t s, int kvdtype, const AttnParams& p, uint32_t T);
+// The same on tcgen05 for float16 caches (err: device word that gets bit 4 when a bounded wait gave up).
+bool attn_prefill_umma_supported(int kvdtype, const AttnParams& p, uint32_t T);
+cudaError_t launch_attn_prefill_umma(cudaStream_t s, const AttnParams& p, uint32_t T, uint32_t* err);
 
 // Long-context variant for a float16 cache (d = 64 or 128, four query heads per CTA): K and V staged through
 // shared-memory rings by 2-D tile copies. The two tile descriptors (one K, one V per layer) are built on the host.

@@ -1,6 +1,9 @@
-"""Tiles of the prompt kernels at their edges: products over pairs of SMs, against float64 products of the same operands."""
+"""Tiles of the prompt kernels at their edges: products over pairs of SMs against float64 products of the same operands, attention in
+tensor memory against the warp-level kernel of the same arithmetic."""
 import numpy as np
 import pytest
+
+from nfai_b200 import create_synthetic_model, LlamaModelFactory, synth
 
 from .gpu_util import call, host, ptr, rel_err
 
@@ -24,3 +27,39 @@ def test_pair_tiles(cuda_ctx, M, N, K):
     got = host(C)
     assert np.isfinite(got).all()
     assert rel_err(got, want) < 1e-5  # float32 sums of at most 200 products: 200 * 2^-24
+
+
+@pytest.fixture(scope="module")
+def factory():
+    f = LlamaModelFactory(0)
+    yield f
+    f.Dispose()
+
+
+@pytest.mark.parametrize("position,tokens", [(0, 257),     # the shortest walk taken: a third tile of one position
+                                             (248, 9),     # the fewest tokens, rows of one CTA only in part
+                                             (255, 130),
+                                             (383, 33),    # the last position of a tile is the first token's own
+                                             (1000, 517)])
+@pytest.mark.parametrize("heads,kv_heads,d", [(8, 2, 64), (6, 2, 128), (3, 3, 64), (5, 1, 128)])
+def test_attention_tiles(factory, monkeypatch, heads, kv_heads, d, position, tokens):
+    """Rows behind the last token are NaN; some keys score far above all before them, so that sums are rescaled on the way."""
+    cfg = synth.get_config("s3", qH=heads, kvH=kv_heads, d=d, H=heads * d, gain_std=0.1)
+    m = create_synthetic_model(cfg, 1664, factory=factory, kv_dtype="f16")
+    rng = np.random.default_rng(position + tokens + heads)
+    for layer in range(cfg.L):
+        k, v = (rng.standard_normal((1664, cfg.kvDim), dtype=np.float32) for _ in "kv")
+        k[100:120] *= 8
+        k[200:210] *= 30
+        k[position:] = v[position:] = np.nan
+        m.write_kv_range(layer, 0, k, v)
+    ids = synth.prompt_ids(cfg, tokens, 7)
+    out = {}
+    for kind in ("1", "2"):
+        monkeypatch.setenv("NFAI_PREFILL_ATTN", kind)
+        m.set_position(position)
+        out[kind] = m.prefill(ids)[0], m.read_hidden(0), m.read_hidden(1)
+    m.Dispose()
+    for a, b in zip(out["2"], out["1"]):
+        assert np.isfinite(a).all()
+        assert rel_err(a, b) < 2e-3  # (float32 sums in another order, rounded to float16 between the kernels: a few 2^-11)
