@@ -871,12 +871,20 @@ int nfai_model_finalize(nfai_model* m) {
   // batched prompt workspace
   const bool want_pf = hp.weight_dtype == NFAI_F16 && env_int("NFAI_PREFILL_GEMM", 1) != 0 &&
                        hp.H % 8 == 0 && m->qDimL % 8 == 0 && m->Fl % 8 == 0;
-  // tokens per pass of the batched prompt path: long passes amortise ~130 launches per pass and fill the GEMM grids
-  uint32_t pf_want = (uint32_t)env_int("NFAI_PREFILL_CHUNK", 2048);
-  if (pf_want < 8) pf_want = 8;
-  if (pf_want > 8192) pf_want = 8192;
-  const uint32_t pfc = want_pf ? (hp.ctx < pf_want ? hp.ctx : pf_want) : 0;
   const uint32_t amax = hp.H > m->qDimL ? hp.H : m->qDimL;
+  // Tokens per pass of the batched prompt path: long passes amortise ~130 launches per pass and fill the GEMM grids. With sm / 4
+  // row tiles of 256 tokens (9 472) every matrix whose columns are a multiple of 512 makes whole waves of the sm / 2 pairs of
+  // SMs, and so do the 128-row tiles of the attention; a pass costs its tokens times the row below (90 KB for the 8B
+  // architecture), so 2 048 where that does not fit beside the rest, and under tensor parallelism, where ranks take equal passes.
+  const size_t pf_row = (size_t)hp.H * 8 + (size_t)amax * 2 + (size_t)m->qDimL * 6 + (size_t)m->Fl * 2 + 4;
+  const uint32_t pf_long = sm_count() / 4 * 256;
+  size_t mem_free = 0, mem_all = 0;
+  CU(c, cudaMemGetInfo(&mem_free, &mem_all));
+  const bool roomy = c->world == 1 && mem_free > arena.off + pf_row * pf_long + ((size_t)1 << 30);
+  uint32_t pf_want = (uint32_t)env_int("NFAI_PREFILL_CHUNK", roomy ? (int)pf_long : 2048);
+  if (pf_want < 8) pf_want = 8;
+  if (pf_want > 16384) pf_want = 16384;
+  const uint32_t pfc = want_pf ? (hp.ctx < pf_want ? hp.ctx : pf_want) : 0;
   const size_t o_px0 = take((size_t)pfc * hp.H * 4);
   const size_t o_px1 = take((size_t)pfc * hp.H * 4);
   const size_t o_pa = take((size_t)pfc * amax * 2);
