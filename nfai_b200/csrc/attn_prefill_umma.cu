@@ -18,7 +18,8 @@
 // Precision as in attn_prefill_tc.cu: q (scaled) and weights rounded to float16 for the products, everything else float32.
 //
 // Against the warp-level kernel of attn_prefill_tc.cu (us): 2011 tokens, 32 heads of 64: 37 against 68; 24 heads of 128: 48
-// against 98; 2048 behind 28000, 32 heads of 64: 742 against 1783 (656 TFLOP/s); 9472 behind 18944: 2353 against 5771 (781).
+// against 98 (46 with elected issue); 2048 behind 28000, 32 heads of 64: 732 against 1783 (665 TFLOP/s); 9472 behind 18944: 2317
+// against 5771 (793).
 //
 // Reference arithmetic replaced: AttentionScoreCalculationShader.cs:170-205, AttentionSoftmaxShader.cs:145-177,
 // AttentionWeightedValueSumShader.cs:181-215, applied once per prompt token by LlamaModel.cs:103-126.
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(kUThreads, 2) attn_prefill_umma_kernel(const _
   uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * SM::kSlots + 5);
   const uint32_t full0 = s_u32(bars), empty0 = s_u32(bars + SM::kSlots), q_ready = s_u32(bars + 2 * SM::kSlots), s_ready = q_ready + 8,
                  s_free = q_ready + 16, p_ready = q_ready + 24, pv_done = q_ready + 32;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  // (warp: uniform)
   if (tid == 0) {
     for (uint32_t i = 0; i < SM::kSlots; ++i) {
       bar_init(full0 + 8 * i, 1);
@@ -145,46 +146,46 @@ __global__ void __launch_bounds__(kUThreads, 2) attn_prefill_umma_kernel(const _
   bool ok = true;
 
   if (warp == 8) {
-    if (lane == 0) {
-      uint32_t j = 0;
-      auto load = [&](const CUtensorMap* map, uint32_t it) {
-        const uint32_t s = j % SM::kSlots;
-        if (j >= SM::kSlots && !bar_wait(empty0 + 8 * s, (j / SM::kSlots - 1) & 1)) return ok = false;
+    uint32_t j = 0;
+    auto load = [&](const CUtensorMap* map, uint32_t it) {
+      const uint32_t s = j % SM::kSlots;
+      if (j >= SM::kSlots && !warp_wait(empty0 + 8 * s, (j / SM::kSlots - 1) & 1)) return ok = false;
+      if (elect_one()) {
         bar_expect_tx(full0 + 8 * s, SM::kTile);
 #pragma unroll
         for (uint32_t b = 0; b < D / 64; ++b)
           tma_load_2d(s_u32(sm) + SM::kQ + s * SM::kTile + b * (kUN * 128), map, (int)(g * D + b * 64), (int)(it * kUN), full0 + 8 * s);
-        ++j;
-        return true;
-      };
-      if constexpr (kAhead) {
-        load(&mapK, 0);
-        for (uint32_t it = 0; it < n && ok; ++it) {
-          if (it + 1 < n && !load(&mapK, it + 1)) break;
-          if (!load(&mapV, it)) break;
-        }
-      } else {
-        for (uint32_t it = 0; it < n && ok; ++it)
-          if (!load(&mapK, it) || !load(&mapV, it)) break;
       }
+      ++j;
+      return true;
+    };
+    if constexpr (kAhead) {
+      load(&mapK, 0);
+      for (uint32_t it = 0; it < n && ok; ++it) {
+        if (it + 1 < n && !load(&mapK, it + 1)) break;
+        if (!load(&mapV, it)) break;
+      }
+    } else {
+      for (uint32_t it = 0; it < n && ok; ++it)
+        if (!load(&mapK, it) || !load(&mapV, it)) break;
     }
   } else if (warp == 9) {
-    if (lane == 0) {
-      // float16 operands, float32 sums; A along K in both products; B along K (K tile) or along N (V tile)
-      constexpr uint32_t idesc_s = (1u << 4) | ((kUN >> 3) << 17) | ((kUM >> 4) << 24);
-      constexpr uint32_t idesc_o = (1u << 4) | (1u << 16) | ((uint32_t)(D >> 3) << 17) | ((kUM >> 4) << 24);
-      const uint32_t q_s = s_u32(sm);
-      uint32_t j = 0;
-      auto slot = [&](uint32_t& s) {  // wait for the next tile
-        s = j % SM::kSlots;
-        ok = bar_wait(full0 + 8 * s, (j / SM::kSlots) & 1);
-        fence_after();
-        ++j;
-        return ok;
-      };
-      auto scores = [&]() {
-        uint32_t s;
-        if (!slot(s)) return false;
+    // float16 operands, float32 sums; A along K in both products; B along K (K tile) or along N (V tile)
+    constexpr uint32_t idesc_s = (1u << 4) | ((kUN >> 3) << 17) | ((kUM >> 4) << 24);
+    constexpr uint32_t idesc_o = (1u << 4) | (1u << 16) | ((uint32_t)(D >> 3) << 17) | ((kUM >> 4) << 24);
+    const uint32_t q_s = s_u32(sm);
+    uint32_t j = 0;
+    auto slot = [&](uint32_t& s) {  // wait for the next tile
+      s = j % SM::kSlots;
+      ok = warp_wait(full0 + 8 * s, (j / SM::kSlots) & 1);
+      fence_after();
+      ++j;
+      return ok;
+    };
+    auto scores = [&]() {
+      uint32_t s;
+      if (!slot(s)) return false;
+      if (elect_one()) {
         const uint32_t k_s = q_s + SM::kQ + s * SM::kTile;
 #pragma unroll
         for (uint32_t kk = 0; kk < D / 16; ++kk) {
@@ -193,30 +194,32 @@ __global__ void __launch_bounds__(kUThreads, 2) attn_prefill_umma_kernel(const _
         }
         umma_commit(empty0 + 8 * s);
         umma_commit(s_ready);
-        return true;
-      };
-      ok = bar_wait(q_ready, 0);
-      fence_after();
-      if (ok) scores();
-      for (uint32_t it = 0; it < n && ok; ++it) {
-        if (kAhead && it + 1 < n) {
-          if (!(ok = bar_wait(s_free, it & 1))) break;
-          fence_after();
-          if (!scores()) break;
-        }
-        if (!(ok = bar_wait(p_ready, it & 1))) break;
+      }
+      return true;
+    };
+    ok = warp_wait(q_ready, 0);
+    fence_after();
+    if (ok) scores();
+    for (uint32_t it = 0; it < n && ok; ++it) {
+      if (kAhead && it + 1 < n) {
+        if (!(ok = warp_wait(s_free, it & 1))) break;
         fence_after();
-        uint32_t s;
-        if (!slot(s)) break;
+        if (!scores()) break;
+      }
+      if (!(ok = warp_wait(p_ready, it & 1))) break;
+      fence_after();
+      uint32_t s;
+      if (!slot(s)) break;
+      if (elect_one()) {
         const uint32_t v_s = q_s + SM::kQ + s * SM::kTile;
 #pragma unroll
         for (uint32_t kk = 0; kk < kUN / 16; ++kk)
           umma_f16_ta(tmem + kO, tmem + kP + kk * 8, smem_desc_mn_sw128(v_s + kk * 2048, kUN * 128), idesc_o, (it | kk) != 0);
         umma_commit(empty0 + 8 * s);
         umma_commit(pv_done);
-        // (the weights lie where the next scores go: products of one thread run in their order)
-        if (!kAhead && it + 1 < n && !scores()) break;
       }
+      // (the weights lie where the next scores go: products of one thread run in their order)
+      if (!kAhead && it + 1 < n && !scores()) break;
     }
   } else {
     const uint32_t qDim = p.qH * D;
@@ -315,10 +318,12 @@ __global__ void __launch_bounds__(kUThreads, 2) attn_prefill_umma_kernel(const _
           }
         };
         weights(0);
+        if (!kAhead) fence_before();  // (the other warp's scores may lie where this one's weights go: both have read theirs now)
         if (either(top > m + kGrowth) && !raise) {
           raise = true;
           continue;
         }
+        if (!kAhead) fence_after();
         if (kAhead) {
           fence_before();
           __syncwarp();

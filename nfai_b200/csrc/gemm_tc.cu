@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_cons
   // bars[0..STAGES) full, [STAGES..2*STAGES) empty, [2*STAGES] accumulator ready; then the TMEM base address word
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 1);
   const uint32_t full0 = s_u32(bars), empty0 = s_u32(bars + STAGES), accbar = s_u32(bars + 2 * STAGES);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // (uniform)
   const uint32_t m0 = blockIdx.y * kBM, n0 = blockIdx.x * BN;
   // this CTA's share of the K tiles (split-K: blockIdx.z of gridDim.z; every share holds at least one tile)
   const uint32_t KT_all = (K + kBK - 1) / kBK;
@@ -299,12 +299,12 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_cons
   pdl_wait();
 
   if (warp == 0) {
-    if (lane == 0) {
-      for (uint32_t kt = 0; kt < KT; ++kt) {
-        const uint32_t s = kt % STAGES;
-        if (kt >= (uint32_t)STAGES) {
-          if (!bar_wait(empty0 + 8 * s, ((kt / STAGES) - 1) & 1)) { ok = false; break; }
-        }
+    for (uint32_t kt = 0; kt < KT; ++kt) {
+      const uint32_t s = kt % STAGES;
+      if (kt >= (uint32_t)STAGES) {
+        if (!(ok = warp_wait(empty0 + 8 * s, ((kt / STAGES) - 1) & 1))) break;
+      }
+      if (elect_one()) {
         const uint32_t a_dst = s_u32(gsm + s * SM::kStage), b_dst = a_dst + SM::kABytes;
         bar_expect_tx(full0 + 8 * s, SM::kABytes + SM::kBBytes);
         tma_load_2d(a_dst, &mapA, (int)((kt0 + kt) * kBK), (int)m0, full0 + 8 * s);
@@ -312,21 +312,21 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // instruction descriptor: D float32, A and B of one 16-bit type (0 = float16, 1 = bfloat16), both K-major, N = BN, M = 128
-      const uint32_t idesc = (1u << 4) | (ep.operands_bf16 << 7) | (ep.operands_bf16 << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-      for (uint32_t kt = 0; kt < KT; ++kt) {
-        const uint32_t s = kt % STAGES;
-        if (!bar_wait(full0 + 8 * s, (kt / STAGES) & 1)) { ok = false; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // instruction descriptor: D float32, A and B of one 16-bit type (0 = float16, 1 = bfloat16), both K-major, N = BN, M = 128
+    const uint32_t idesc = (1u << 4) | (ep.operands_bf16 << 7) | (ep.operands_bf16 << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+    for (uint32_t kt = 0; kt < KT; ++kt) {
+      const uint32_t s = kt % STAGES;
+      if (!(ok = warp_wait(full0 + 8 * s, (kt / STAGES) & 1))) break;
+      fence_after();
+      if (elect_one()) {
         const uint32_t a_s = s_u32(gsm + s * SM::kStage), b_s = a_s + SM::kABytes;
 #pragma unroll
         for (int k = 0; k < kBK / 16; ++k) {
           umma_f16(tmem_base, smem_desc_sw128(a_s + k * 32), smem_desc_sw128(b_s + k * 32), idesc, (kt | (uint32_t)k) != 0);
         }
         umma_commit(empty0 + 8 * s);  // arrives when the MMAs above have finished reading the stage
+        if (kt + 1 == KT) umma_commit(accbar);
       }
-      if (ok) umma_commit(accbar);
     }
   } else {
     // epilogue warps 2..5: warp w may touch tensor-memory lanes 32*(w%4) .. +31
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_grouped_kernel(const __
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   const uint32_t full0 = s_u32(bars), empty0 = s_u32(bars + STAGES), tfull0 = s_u32(bars + 2 * STAGES),
                  tempty0 = s_u32(bars + 2 * STAGES + 2);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // (uniform)
   const uint32_t KT = (K + kBK - 1) / kBK;
   const uint32_t ntiles = (N + kPBN - 1) / kPBN;
 
@@ -432,15 +432,15 @@ __global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_grouped_kernel(const __
   };
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t it = 0;
-      for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        const Tile at = tile_at(tile);
-        for (uint32_t kt = 0; kt < KT; ++kt, ++it) {
-          const uint32_t s = it % STAGES;
-          if (it >= (uint32_t)STAGES) {
-            if (!bar_wait(empty0 + 8 * s, ((it / STAGES) - 1) & 1)) { ok = false; break; }
-          }
+    uint32_t it = 0;
+    for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+      const Tile at = tile_at(tile);
+      for (uint32_t kt = 0; kt < KT; ++kt, ++it) {
+        const uint32_t s = it % STAGES;
+        if (it >= (uint32_t)STAGES) {
+          if (!(ok = warp_wait(empty0 + 8 * s, ((it / STAGES) - 1) & 1))) break;
+        }
+        if (elect_one()) {
           const uint32_t a_dst = s_u32(gsm + s * SM::kStage), b_dst = a_dst + SM::kABytes;
           bar_expect_tx(full0 + 8 * s, SM::kABytes + SM::kBBytes);
           tma_load_2d(a_dst, &mapA, (int)(kt * kBK), (int)at.m0, full0 + 8 * s);
@@ -449,28 +449,28 @@ __global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_grouped_kernel(const __
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (ep.operands_bf16 << 7) | (ep.operands_bf16 << 10) | ((uint32_t)(kPBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-      uint32_t it = 0, i = 0;
-      for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++i) {
-        const uint32_t acc = i & 1;
-        if (i >= 2) {  // the epilogue must have drained this half of tensor memory (tile i - 2)
-          if (!bar_wait(tempty0 + 8 * acc, ((i >> 1) - 1) & 1)) { ok = false; break; }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        }
-        const uint32_t d = tmem_base + acc * (uint32_t)kPBN;
-        for (uint32_t kt = 0; kt < KT; ++kt, ++it) {
-          const uint32_t s = it % STAGES;
-          if (!bar_wait(full0 + 8 * s, (it / STAGES) & 1)) { ok = false; break; }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t idesc = (1u << 4) | (ep.operands_bf16 << 7) | (ep.operands_bf16 << 10) | ((uint32_t)(kPBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+    uint32_t it = 0, i = 0;
+    for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++i) {
+      const uint32_t acc = i & 1;
+      if (i >= 2) {  // the epilogue must have drained this half of tensor memory (tile i - 2)
+        if (!(ok = warp_wait(tempty0 + 8 * acc, ((i >> 1) - 1) & 1))) break;
+        fence_after();
+      }
+      const uint32_t d = tmem_base + acc * (uint32_t)kPBN;
+      for (uint32_t kt = 0; kt < KT; ++kt, ++it) {
+        const uint32_t s = it % STAGES;
+        if (!(ok = warp_wait(full0 + 8 * s, (it / STAGES) & 1))) break;
+        fence_after();
+        if (elect_one()) {
           const uint32_t a_s = s_u32(gsm + s * SM::kStage), b_s = a_s + SM::kABytes;
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k) {
             umma_f16(d, smem_desc_sw128(a_s + k * 32), smem_desc_sw128(b_s + k * 32), idesc, (kt | (uint32_t)k) != 0);
           }
           umma_commit(empty0 + 8 * s);
+          if (kt + 1 == KT) umma_commit(tfull0 + 8 * acc);
         }
-        if (ok) umma_commit(tfull0 + 8 * acc);
       }
     }
   } else {
@@ -509,8 +509,8 @@ __global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_grouped_kernel(const __
 // a tile runs beside the products of the next.
 // Each CTA's warp 0 copies its own operands and counts them on the first CTA's barrier; the first CTA's warp 1 issues the
 // products of both; epilogues by eight warps of each CTA, its rows. Measured against a 128 x 256 tile per SM (us, 1.9 GHz):
-// 2011 x 16384 x 2048 112 against 120, 2011 x 3072 x 8192 94 and 103, 9472 x 16384 x 2048 496 and 528, 1024 x 28672 x 4096 192
-// and 208, 2011 x 2048 x 2048 22.6 and 21.8.
+// 2011 x 16384 x 2048 105 against 120, 2011 x 3072 x 8192 78 and 103, 2011 x 5120 x 3072 50 and 65, 9472 x 16384 x 2048 470 and
+// 528, 2011 x 2048 x 2048 18.4 and 21.8.
 constexpr int kPairStages = 6;
 struct PairSmem {
   static constexpr uint32_t kABytes = kBM * kBK * 2;
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_pair_kernel(const __gri
   // as in the grouped kernel; "full" and "accumulator empty" count in the first CTA, the others in both
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   const uint32_t full0 = s_u32(bars), empty0 = s_u32(bars + STAGES), tfull0 = s_u32(bars + 2 * STAGES), tempty0 = s_u32(bars + 2 * STAGES + 2);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // (uniform)
   const uint32_t rank = cluster_rank(), KT = (K + kBK - 1) / kBK;
   const uint32_t mtiles = (M + 2 * kBM - 1) / (2 * kBM), tiles = mtiles * ((N + BN - 1) / BN);
   const uint32_t first = blockIdx.x >> 1, step = gridDim.x >> 1;
@@ -563,16 +563,16 @@ __global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_pair_kernel(const __gri
   pdl_wait();
 
   if (warp == 0) {
-    if (lane == 0) {
-      const uint32_t b_bytes = BN / 2 * kBK * 2;
-      uint32_t it = 0;
-      for (uint32_t tile = first; tile < tiles && ok; tile += step) {
-        const uint32_t m0 = (tile % mtiles) * (2 * kBM) + rank * kBM, w0 = (tile / mtiles) * BN + rank * (BN / 2);
-        for (uint32_t kt = 0; kt < KT; ++kt, ++it) {
-          const uint32_t s = it % STAGES;
-          if (it >= (uint32_t)STAGES) {
-            if (!bar_wait(empty0 + 8 * s, ((it / STAGES) - 1) & 1)) { ok = false; break; }
-          }
+    const uint32_t b_bytes = BN / 2 * kBK * 2;
+    uint32_t it = 0;
+    for (uint32_t tile = first; tile < tiles && ok; tile += step) {
+      const uint32_t m0 = (tile % mtiles) * (2 * kBM) + rank * kBM, w0 = (tile / mtiles) * BN + rank * (BN / 2);
+      for (uint32_t kt = 0; kt < KT; ++kt, ++it) {
+        const uint32_t s = it % STAGES;
+        if (it >= (uint32_t)STAGES) {
+          if (!(ok = warp_wait(empty0 + 8 * s, ((it / STAGES) - 1) & 1))) break;
+        }
+        if (elect_one()) {
           const uint32_t a_dst = s_u32(gsm + s * SM::kStage), b_dst = a_dst + SM::kABytes, full = in_leader(full0 + 8 * s);
           if (rank == 0) bar_expect_tx(full0 + 8 * s, 2 * (SM::kABytes + b_bytes));
           tma_load_2d_pair(a_dst, &mapA, (int)(kt * kBK), (int)m0, full);
@@ -581,27 +581,29 @@ __global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_pair_kernel(const __gri
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       const uint32_t idesc = (1u << 4) | (ep.operands_bf16 << 7) | (ep.operands_bf16 << 10) | ((BN >> 3) << 17) | ((uint32_t)(2 * kBM >> 4) << 24);
       uint32_t it = 0, i = 0;
       for (uint32_t tile = first; tile < tiles && ok; tile += step, ++i) {
         const uint32_t acc = i & 1;
         if (i >= 2) {  // both epilogues must have drained this half of tensor memory
-          if (!bar_wait_cluster(tempty0 + 8 * acc, ((i >> 1) - 1) & 1)) { ok = false; break; }
+          if (!(ok = warp_wait_cluster(tempty0 + 8 * acc, ((i >> 1) - 1) & 1))) break;
           fence_after();
         }
         const uint32_t d = tmem_base + acc * 256u;
         for (uint32_t kt = 0; kt < KT; ++kt, ++it) {
           const uint32_t s = it % STAGES;
-          if (!bar_wait_cluster(full0 + 8 * s, (it / STAGES) & 1)) { ok = false; break; }
+          if (!(ok = warp_wait_cluster(full0 + 8 * s, (it / STAGES) & 1))) break;
           fence_after();
-          const uint32_t a_s = s_u32(gsm + s * SM::kStage), b_s = a_s + SM::kABytes;
+          if (elect_one()) {
+            const uint32_t a_s = s_u32(gsm + s * SM::kStage), b_s = a_s + SM::kABytes;
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k)
-            umma_f16_pair(d, smem_desc_sw128(a_s + k * 32), smem_desc_sw128(b_s + k * 32), idesc, (kt | (uint32_t)k) != 0);
-          umma_commit_pair(empty0 + 8 * s);
+            for (int k = 0; k < kBK / 16; ++k)
+              umma_f16_pair(d, smem_desc_sw128(a_s + k * 32), smem_desc_sw128(b_s + k * 32), idesc, (kt | (uint32_t)k) != 0);
+            umma_commit_pair(empty0 + 8 * s);
+            if (kt + 1 == KT) umma_commit_pair(tfull0 + 8 * acc);
+          }
         }
-        if (ok) umma_commit_pair(tfull0 + 8 * acc);
       }
     }
   } else {
