@@ -6,13 +6,14 @@
 // tolerance, so the fused epilogues below are the same ones the decode GEMVs use (RoPE + cache write, SiLU*up,
 // residual add) applied row by row.
 //
-// Shape of one CTA (192 threads, one 128 x BN output tile):
+// Shape of one CTA (320 threads, one 128 x BN output tile):
 //   warp 0      producer: one lane issues TMA tile loads (A 128x64, W BNx64 halves, 128-byte swizzle) into a ring of
 //               shared-memory stages, completion counted on the stage's "full" mbarrier;
 //   warp 1      MMA: allocates BN tensor-memory columns; one lane waits for a full stage, issues four
 //               tcgen05.mma (K = 16 each) from shared-memory descriptors, and commits to the stage's "empty"
 //               mbarrier so that the producer may refill it; after the last stage it commits to "accumulator ready";
-//   warps 2-5   epilogue: each reads its 32 accumulator rows with tcgen05.ld and applies the epilogue.
+//   warps 2-9   epilogue: two for each quarter of the accumulator's rows (a warp may only read the lanes of its index modulo 4),
+//               taking its column blocks in turn.
 // No cluster-wide delivery is used anywhere. Every mbarrier wait is bounded (one second): on a time-out the role
 // records an error bit and leaves; the tensor memory is released on every path.
 #include <cuda.h>
@@ -37,7 +38,7 @@ using namespace umma;
 
 constexpr int kBM = 128;
 constexpr int kBK = 64;  // halves per stage row = 128 bytes = one swizzle span
-constexpr int kGemmThreads = 192;
+constexpr int kGemmThreads = 64 + 8 * 32;
 constexpr uint32_t kEpiWarp = 32 * 32 * 4;  // an epilogue warp's shared memory
 
 // ---- epilogue of an accumulator tile ------------------------------------------------------------------------------
@@ -45,7 +46,7 @@ constexpr uint32_t kEpiWarp = 32 * 32 * 4;  // an epilogue warp's shared memory
 // shared memory in 16-byte quads (quad j of row r lies at place j ^ (r & 7): neither side conflicts) and comes back with 8 lanes
 // on the 32 columns of a row, 4 rows per instruction, all of it in registers before the first store: 8 wide loads and stores per
 // lane and block. Stores of single columns or pairs from the accumulator's layout touched 32 rows per instruction: 256 x 2048 at
-// K = 64 took 8.0 us, now 3.6; 128 x 16384 x 2048 (67 MB of weights) 34 us.
+// K = 64 took 8.0 us, now 3.6; 128 x 16384 x 2048 (67 MB of weights) 34, now 17.4 (19.5 with gates; 18.2 and 22.8 with four warps).
 
 // Whether every quad of columns that lies below N can be read and written in one piece
 template <int KIND>
@@ -120,7 +121,7 @@ __device__ __forceinline__ bool tile_epilogue(const GemmEpilogue& ep, const uint
       }
     }
   };
-  if (kRows && fit) load_aux(c_first);
+  if (kRows && fit && c_first < blocks) load_aux(c_first);
   bool good = bar_wait(tfull, parity);
   good = __all_sync(0xffffffffu, good);
   if (!good) return false;
@@ -253,11 +254,13 @@ struct GemmSmem {
   static constexpr uint32_t kStage = kABytes + kBBytes;
   static constexpr uint32_t kBarOff = STAGES * kStage;
   static constexpr uint32_t kEpiOff = kBarOff + 256;
-  static constexpr uint32_t kTotal = kEpiOff + 4 * kEpiWarp + 1024;  // slack for the 1024-byte alignment
+  static constexpr uint32_t kTotal = kEpiOff + 8 * kEpiWarp + 1024;  // slack for the 1024-byte alignment
 };
 
-// (KIND: the epilogue; a split stores raw partial sums into [split][M][N], the finishing kernel applies it)
-template <int BN, int STAGES, int KIND>
+// KIND: the epilogue. A split of K over gridDim.z CTAs adds up in one of two ways. REDUCE: those CTAs are a cluster; each leaves
+// its sums in its shared memory and, when all have, adds its share of the rows over the cluster (in split order) and applies the
+// epilogue. Otherwise raw sums go into [split][M][N] and a finishing kernel adds them in the same order.
+template <int BN, int STAGES, int KIND, bool REDUCE>
 __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA,
                                                                const __grid_constant__ CUtensorMap mapW, uint32_t M,
                                                                uint32_t N, uint32_t K, const GemmEpilogue ep,
@@ -329,15 +332,31 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_cons
       }
     }
   } else {
-    // epilogue warps 2..5: warp w may touch tensor-memory lanes 32*(w%4) .. +31
+    // warp w may touch tensor-memory lanes 32*(w%4) .. +31
     const uint32_t lane_grp = (uint32_t)(warp & 3);
     const uint32_t eb = s_u32(gsm + SM::kEpiOff) + (warp - 2) * kEpiWarp;
-    if (gridDim.z > 1) {
+    if constexpr (REDUCE) {  // quad q of row r at place q ^ r (of the row's BN / 4): neither the writes nor the reads conflict
+      ok = __all_sync(0xffffffffu, bar_wait(accbar, 0));
+      if (ok) {
+        fence_after();
+        const uint32_t r = lane_grp * 32 + lane;
+#pragma unroll 1
+        for (uint32_t b = (warp - 2) >> 2; b < BN / 32; b += 2) {
+          uint32_t v[32];
+          tmem_ld(tmem_base + ((lane_grp * 32u) << 16) + b * 32u, v);
+#pragma unroll
+          for (uint32_t q = 0; q < 8; ++q)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(s_u32(gsm) + r * (BN * 4) + (((b * 8 + q) ^ (r & (BN / 4 - 1))) << 4)),
+                         "r"(v[4 * q]), "r"(v[4 * q + 1]), "r"(v[4 * q + 2]), "r"(v[4 * q + 3])
+                         : "memory");
+        }
+      }
+    } else if (gridDim.z > 1) {
       GemmEpilogue part;
       part.out_f32 = ep.scratch + (size_t)blockIdx.z * M * N;
-      ok = tile_epilogue<GEMM_EPI_STORE>(part, m0, M, n0, N, BN / 32, tmem_base, lane_grp, 0, 1, lane, eb, accbar, 0);
+      ok = tile_epilogue<GEMM_EPI_STORE>(part, m0, M, n0, N, BN / 32, tmem_base, lane_grp, (warp - 2) >> 2, 2, lane, eb, accbar, 0);
     } else {
-      ok = tile_epilogue<KIND>(ep, m0, M, n0, N, BN / 32, tmem_base, lane_grp, 0, 1, lane, eb, accbar, 0);
+      ok = tile_epilogue<KIND>(ep, m0, M, n0, N, BN / 32, tmem_base, lane_grp, (warp - 2) >> 2, 2, lane, eb, accbar, 0);
     }
   }
   if (!ok) {
@@ -346,6 +365,27 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_cons
     // tensor memory are released
     for (volatile uint32_t spin = 0; spin < (1u << 20); ++spin) {
     }
+  }
+  if constexpr (REDUCE) {
+    static_assert(BN == 128 && kBM * BN * 4 <= SM::kBarOff, "a lane for each quad, and the sums where the stages were");
+    __syncwarp();
+    cluster_sync();
+    const uint32_t Z = gridDim.z, live = min((uint32_t)kBM, M - m0), per = (live + Z - 1) / Z;
+    const uint32_t end = min(live, (blockIdx.z + 1) * per), n = n0 + lane * 4;
+    for (uint32_t r = blockIdx.z * per + warp; r < end && n < N; r += kGemmThreads / 32) {
+      const uint32_t m = m0 + r, at = s_u32(gsm) + r * (BN * 4) + ((lane ^ (r & 31)) << 4);
+      const float2 aux0 = epilogue_aux<KIND>(ep, m, n, N), aux1 = n + 2 < N ? epilogue_aux<KIND>(ep, m, n + 2, N) : make_float2(0.f, 0.f);
+      float4 part[8];
+#pragma unroll
+      for (uint32_t z = 0; z < 8; ++z) part[z] = z < Z ? ld_cluster(at, z) : make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (uint32_t z = 0; z < 8; ++z) x = make_float4(x.x + part[z].x, x.y + part[z].y, x.z + part[z].z, x.w + part[z].w);
+      epilogue_pair<KIND>(ep, m, n, N, x.x, x.y, aux0);
+      if (n + 2 < N) epilogue_pair<KIND>(ep, m, n + 2, N, x.z, x.w, aux1);
+    }
+    __syncwarp();
+    cluster_sync();  // nobody reads the memory of a CTA that has left
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -720,12 +760,45 @@ bool tile_map16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, u
 
 namespace {
 
+// Clusters of Z CTAs (along a split of K) that run at the same time: a cluster's CTAs share a group of 16 to 18 SMs.
 template <int BN, int STAGES, int KIND>
+uint32_t clusters_at_once(uint32_t Z) {
+  static thread_local int device = -1, known[9] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (device != dev) {
+    for (int& k : known) k = -1;
+    device = dev;
+  }
+  if (known[Z] < 0) {
+    auto kern = gemm_tc_kernel<BN, STAGES, KIND, true>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sm_count() / Z, 1, Z);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = GemmSmem<BN, STAGES>::kTotal;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = Z;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    known[Z] = n;
+  }
+  return (uint32_t)known[Z];
+}
+
+template <int BN, int STAGES, int KIND, bool REDUCE = false>
 cudaError_t launch_bn_kind(cudaStream_t s, const __half* A, const __half* W, uint32_t M, uint32_t N, uint32_t K,
                       const GemmEpilogue& ep, uint32_t* err, uint32_t Z) {
   CUtensorMap mapA, mapW;
   if (!tile_map16(&mapA, A, M, K, kBM) || !tile_map16(&mapW, W, N, K, BN)) return cudaErrorInvalidValue;
-  auto kern = gemm_tc_kernel<BN, STAGES, KIND>;
+  auto kern = gemm_tc_kernel<BN, STAGES, KIND, REDUCE>;
   const size_t smem = GemmSmem<BN, STAGES>::kTotal;
   static thread_local int attr_device = -1;  // the attribute is per device: set it once per (thread, device)
   int dev = 0;
@@ -737,6 +810,7 @@ cudaError_t launch_bn_kind(cudaStream_t s, const __half* A, const __half* W, uin
     attr_device = dev;
   }
   dim3 grid((N + BN - 1) / BN, (M + kBM - 1) / kBM, Z);
+  if constexpr (REDUCE) return launch_pdl_cluster(kern, grid, dim3(kGemmThreads), dim3(1, 1, Z), smem, s, prefill_pdl(), mapA, mapW, M, N, K, ep, err);
   e = launch_pdl(kern, grid, dim3(kGemmThreads), smem, s, prefill_pdl(), mapA, mapW, M, N, K, ep, err);
   if (e != cudaSuccess || Z == 1) return e;
   const size_t pairs = (size_t)M * ((N + 1) / 2);
@@ -761,6 +835,21 @@ template <int BN, int STAGES>
 cudaError_t launch_bn(cudaStream_t s, const __half* A, const __half* W, uint32_t M, uint32_t N, uint32_t K, const GemmEpilogue& ep, uint32_t* err,
                       uint32_t Z = 1) {
   return with_kind(ep.kind, [&](auto kind) { return launch_bn_kind<BN, STAGES, decltype(kind)::value>(s, A, W, M, N, K, ep, err, Z); });
+}
+
+// A split of K, at best Z ways: added up inside clusters when all of them run at once with at least two thirds as many ways, else
+// through memory. (Of 8 CTAs 15 clusters run at once, of 6 22, of 4 33.) 128 x 2048 x 2048: 9.6 us nine ways through memory, 7.8 six
+// ways in clusters; 128 x 3072 x 2048: 9.5 (six), 8.1 (five); 37 x 2048 x 8192: 13.6 (nine), 12.8 (six); 128 x 2048 x 8192: 15.0
+// (nine), 14.4 (six), 16.7 (four).
+cudaError_t launch_split(cudaStream_t s, const __half* A, const __half* W, uint32_t M, uint32_t N, uint32_t K, const GemmEpilogue& ep, uint32_t* err,
+                         uint32_t Z) {
+  return with_kind(ep.kind, [&](auto kind) {
+    constexpr int KIND = decltype(kind)::value;
+    const uint32_t tiles = ((M + kBM - 1) / kBM) * ((N + 127) / 128);
+    for (uint32_t z = Z < 8 ? Z : 8; z > 1 && z * 3 >= Z * 2; --z)
+      if (clusters_at_once<128, 4, KIND>(z) >= tiles) return launch_bn_kind<128, 4, KIND, true>(s, A, W, M, N, K, ep, err, z);
+    return launch_bn_kind<128, 4, KIND>(s, A, W, M, N, K, ep, err, Z);
+  });
 }
 
 template <int KIND>
@@ -813,7 +902,7 @@ cudaError_t launch_pair(cudaStream_t s, const __half* A, const __half* W, uint32
     attr_device = dev;
   }
   const uint32_t tiles = (M + 2 * kBM - 1) / (2 * kBM) * ((N + BN - 1) / BN), pairs = sm_count() / 2;
-  return launch_pdl_cluster(kern, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kPThreadsGemm), 2, PairSmem::kTotal, s, prefill_pdl(), mapA, mapW,
+  return launch_pdl_cluster(kern, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kPThreadsGemm), dim3(2), PairSmem::kTotal, s, prefill_pdl(), mapA, mapW,
                             M, N, K, BN, ep, err);
 }
 
@@ -844,7 +933,7 @@ cudaError_t launch_gemm_tc(cudaStream_t s, const __half* A, const __half* W, uin
   if (ep.scratch) {
     uint32_t Z = gemm_tc_splits(M, N, K);
     while (Z > 1 && (size_t)Z * M * N > ep.scratch_floats) --Z;
-    if (Z > 1) return launch_bn<128, 4>(s, A, W, M, N, K, ep, err, Z);
+    if (Z > 1) return launch_split(s, A, W, M, N, K, ep, err, Z);
   }
   if (mtiles * ((N + 127) / 128) >= 120) return launch_bn<128, 4>(s, A, W, M, N, K, ep, err);
   if (mtiles * ((N + 63) / 64) >= 120) return launch_bn<64, 6>(s, A, W, M, N, K, ep, err);

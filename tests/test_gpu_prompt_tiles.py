@@ -29,6 +29,20 @@ def test_pair_tiles(cuda_ctx, M, N, K):
     assert rel_err(got, want) < 1e-5  # float32 sums of at most 200 products: 200 * 2^-24
 
 
+@pytest.mark.parametrize("M,N,K", [(128, 2048, 2048), (37, 3072, 2048), (1, 2048, 512), (129, 1026, 520),  # rows that do not divide by the cluster
+                                   (16, 2051, 1024), (256, 2048, 1032), (512, 2048, 4096), (70, 130, 4096)])  # the last through memory
+def test_split_tiles(cuda_ctx, M, N, K):
+    """K divided over the CTAs of a cluster, or over more than fit into one: against a float64 product."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    A = (torch.randn(M, K, generator=g, device="cuda") * 0.5).half()
+    W = (torch.randn(N, K, generator=g, device="cuda") * 0.05).half()
+    C = torch.full((M, N), float("nan"), device="cuda")
+    call(cuda_ctx, "nfai_op_gemm_f16", ptr(A), ptr(W), M, N, K, ptr(C))
+    got = host(C)
+    assert np.isfinite(got).all()
+    assert rel_err(got, (A.double() @ W.double().T).cpu().numpy()) < 1e-4  # float32 sums of up to 4096 products
+
+
 @pytest.fixture(scope="module")
 def factory():
     f = LlamaModelFactory(0)
