@@ -1036,8 +1036,8 @@ static int prefill_batched(nfai_model* m, const uint32_t* tokens, int n) {
       AttnParams a;
       a.q = m->pfQ; a.kcache = kcl; a.vcache = vcl; a.qH = m->qHl; a.kvH = m->kvHl; a.d = hp.d;
       a.seq_imm = pos0 + 1; a.out_half = m->pfAO;
-      const int attn_kind = env_int("NFAI_PREFILL_ATTN", 2);  // 0: token at a time, 1: warp-level tensor cores only
-      if (attn_kind >= 2 && attn_prefill_umma_supported(kvdt, a, T)) CU(c, launch_attn_prefill_umma(s, a, T, err));
+      const int attn_kind = env_int("NFAI_PREFILL_ATTN", 1);  // 0: token at a time, 2: warp-level tensor cores only
+      if (attn_kind != 0 && attn_kind != 2 && attn_prefill_umma_supported(kvdt, a, T)) CU(c, launch_attn_prefill_umma(s, a, T, err));
       else if (attn_prefill_tc_supported(hp.d) && attn_kind != 0) CU(c, launch_attn_prefill_tc(s, kvdt, a, T));
       else CU(c, launch_attn_prefill(s, kvdt, a, T));
       // Tensor parallel: the O and down GEMMs produce this rank's partial [T][H]; rank 0 adds the residual into its

@@ -14,7 +14,7 @@
 //               mbarrier so that the producer may refill it; after the last stage it commits to "accumulator ready";
 //   warps 2-9   epilogue: two for each quarter of the accumulator's rows (a warp may only read the lanes of its index modulo 4),
 //               taking its column blocks in turn.
-// No cluster-wide delivery is used anywhere. Every mbarrier wait is bounded (one second): on a time-out the role
+// Larger products: pairs of CTAs (below). No tile copy is delivered to more than one CTA. Every mbarrier wait is bounded (one second): on a time-out the role
 // records an error bit and leaves; the tensor memory is released on every path.
 #include <cuda.h>
 
