@@ -43,6 +43,24 @@ def test_split_tiles(cuda_ctx, M, N, K):
     assert rel_err(got, (A.double() @ W.double().T).cpu().numpy()) < 1e-4  # float32 sums of up to 4096 products
 
 
+@pytest.mark.parametrize("M,N,K", [(1000, 2012, 136), (1000, 2010, 72),                  # tiles of 128 columns
+                                   (640, 2532, 136), (640, 2550, 200),                   # of 64
+                                   (100, 516, 64), (77, 518, 64), (33, 77, 64),          # of 32
+                                   (45, 132, 1024), (70, 130, 1024), (128, 1028, 1024),  # split, through memory and in clusters
+                                   (1537, 4100, 136), (1537, 4098, 136)])                # pairs
+def test_columns_that_end_inside_a_block(cuda_ctx, M, N, K):
+    """The last block of 32 columns is live in some of a warp's lanes only (in quads and in pairs), in every kernel, mostly with dead
+    blocks behind it; nothing is written beyond the product."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    A = (torch.randn(M, K, generator=g, device="cuda") * 0.5).half()
+    W = (torch.randn(N, K, generator=g, device="cuda") * 0.05).half()
+    C = torch.full((M * N + 256,), float("nan"), device="cuda")
+    call(cuda_ctx, "nfai_op_gemm_f16", ptr(A), ptr(W), M, N, K, ptr(C))
+    got = host(C)
+    assert np.isnan(got[M * N:]).all() and np.isfinite(got[:M * N]).all()
+    assert rel_err(got[:M * N].reshape(M, N), (A.double() @ W.double().T).cpu().numpy()) < K * 2.0 ** -24
+
+
 @pytest.fixture(scope="module")
 def factory():
     f = LlamaModelFactory(0)
