@@ -169,6 +169,7 @@ __global__ void __launch_bounds__(kUThreads, 2) attn_prefill_umma_kernel(const _
       for (uint32_t it = 0; it < n && ok; ++it)
         if (!load(&mapK, it) || !load(&mapV, it)) break;
     }
+    if (ok) ok = drain_ring<SM::kSlots>(empty0, j);
   } else if (warp == 9) {
     // float16 operands, float32 sums; A along K in both products; B along K (K tile) or along N (V tile)
     constexpr uint32_t idesc_s = (1u << 4) | ((kUN >> 3) << 17) | ((kUM >> 4) << 24);

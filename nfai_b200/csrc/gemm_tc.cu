@@ -314,6 +314,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_cons
         tma_load_2d(b_dst, &mapW, (int)((kt0 + kt) * kBK), (int)n0, full0 + 8 * s);
       }
     }
+    if (ok) ok = drain_ring<STAGES>(empty0, KT);
   } else if (warp == 1) {
     // instruction descriptor: D float32, A and B of one 16-bit type (0 = float16, 1 = bfloat16), both K-major, N = BN, M = 128
     const uint32_t idesc = (1u << 4) | (ep.operands_bf16 << 7) | (ep.operands_bf16 << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
@@ -488,6 +489,7 @@ __global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_grouped_kernel(const __
         }
       }
     }
+    if (ok) ok = drain_ring<STAGES>(empty0, it);
   } else if (warp == 1) {
     const uint32_t idesc = (1u << 4) | (ep.operands_bf16 << 7) | (ep.operands_bf16 << 10) | ((uint32_t)(kPBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
     uint32_t it = 0, i = 0;
@@ -620,6 +622,7 @@ __global__ void __launch_bounds__(kPThreadsGemm) gemm_tc_pair_kernel(const __gri
         }
       }
     }
+    if (ok) ok = drain_ring<STAGES>(empty0, it);
   } else if (warp == 1) {
     if (rank == 0) {
       const uint32_t idesc = (1u << 4) | (ep.operands_bf16 << 7) | (ep.operands_bf16 << 10) | ((BN >> 3) << 17) | ((uint32_t)(2 * kBM >> 4) << 24);

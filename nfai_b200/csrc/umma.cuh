@@ -90,6 +90,17 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, bar_wait(bar, parity)); }
 __device__ __forceinline__ bool warp_wait_cluster(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, bar_wait_cluster(bar, parity)); }
 
+// A producer's last step after `n` tiles through a ring of STAGES slots: the products' arrivals on the last slots' "empty" barriers,
+// for which no further copy waits. They come from the tensor pipe, in a pair from the other CTA's, and a later arrival on another
+// barrier does not say that they are there; a CTA must not leave (and its memory go to the next kernel) before they are. Costs
+// nothing: the epilogue of the last tile takes longer.
+template <uint32_t STAGES>
+__device__ __forceinline__ bool drain_ring(uint32_t empty0, uint32_t n) {
+  for (uint32_t j = n > STAGES ? n - STAGES : 0; j < n; ++j)
+    if (!warp_wait(empty0 + 8 * (j % STAGES), (j / STAGES) & 1)) return false;
+  return true;
+}
+
 // Shared-memory matrix descriptor: K-major tile, 128-byte swizzle, rows of 128 bytes, 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
   uint64_t d = 0;

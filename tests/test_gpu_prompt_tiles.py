@@ -95,3 +95,20 @@ def test_attention_tiles(factory, monkeypatch, heads, kv_heads, d, position, tok
     for a, b in zip(out["1"], out["2"]):
         assert np.isfinite(a).all()
         assert rel_err(a, b) < 2e-3  # (float32 sums in another order, rounded to float16 between the kernels: a few 2^-11)
+
+
+@pytest.mark.parametrize("key,tokens", [("s1", 1601), ("s2", 300), ("s1", 37)])
+def test_repeated_prompts_agree_to_the_bit(factory, key, tokens):
+    """Kernels of every kind right behind one another (the next one's set-up runs beside the last one's end): what one leaves in
+    flight would show in another's barriers or tiles."""
+    cfg = synth.get_config(key, gain_std=0.1)
+    m = create_synthetic_model(cfg, tokens, factory=factory)
+    ids = synth.prompt_ids(cfg, tokens, 3)
+    first = None
+    for _ in range(8):
+        m.reset()
+        got = [m.prefill(ids)[0]] + [m.read_hidden(l) for l in range(cfg.L)] + [a for l in range(cfg.L) for a in m.read_kv(l, tokens // 2)]
+        assert all(np.isfinite(a).all() for a in got)
+        first = first or got
+        assert all(np.array_equal(a, b) for a, b in zip(got, first))
+    m.Dispose()
