@@ -874,29 +874,42 @@ int nfai_model_finalize(nfai_model* m) {
   const uint32_t amax = hp.H > m->qDimL ? hp.H : m->qDimL;
   // Tokens per pass of the batched prompt path: long passes amortise ~130 launches per pass and fill the GEMM grids. With sm / 4
   // row tiles of 256 tokens (9 472) every matrix whose columns are a multiple of 512 makes whole waves of the sm / 2 pairs of
-  // SMs, and so do the 128-row tiles of the attention; a pass costs its tokens times the row below (90 KB for the 8B
-  // architecture), so 2 048 where that does not fit beside the rest, and under tensor parallelism, where ranks take equal passes.
+  // SMs, and so do the 128-row tiles of the attention. A pass costs its tokens times the row below (90 KB for the 8B
+  // architecture): 2 048 tokens where the long one would take more than a 64th of the device's memory, and under tensor
+  // parallelism, where ranks take equal passes. The length decides in which order sums are added, so it follows from the model,
+  // the context and the device and not from what else is loaded; only a load that would fail otherwise gets 2 048 instead.
   const size_t pf_row = (size_t)hp.H * 8 + (size_t)amax * 2 + (size_t)m->qDimL * 6 + (size_t)m->Fl * 2 + 4;
+  constexpr uint32_t kShortPass = 2048;
   const uint32_t pf_long = sm_count() / 4 * 256;
   size_t mem_free = 0, mem_all = 0;
   CU(c, cudaMemGetInfo(&mem_free, &mem_all));
-  const bool roomy = c->world == 1 && mem_free > arena.off + pf_row * pf_long + ((size_t)1 << 30);
-  uint32_t pf_want = (uint32_t)env_int("NFAI_PREFILL_CHUNK", roomy ? (int)pf_long : 2048);
+  const bool roomy = c->world == 1 && pf_row * std::min(hp.ctx, pf_long) <= mem_all / 64;
+  uint32_t pf_want = (uint32_t)env_int("NFAI_PREFILL_CHUNK", roomy ? (int)pf_long : (int)kShortPass);
   if (pf_want < 8) pf_want = 8;
   if (pf_want > 16384) pf_want = 16384;
-  const uint32_t pfc = want_pf ? (hp.ctx < pf_want ? hp.ctx : pf_want) : 0;
-  const size_t o_px0 = take((size_t)pfc * hp.H * 4);
-  const size_t o_px1 = take((size_t)pfc * hp.H * 4);
-  const size_t o_pa = take((size_t)pfc * amax * 2);
-  const size_t o_pq = take((size_t)pfc * m->qDimL * 4);
-  const size_t o_pao = take((size_t)pfc * m->qDimL * 2);
-  const size_t o_ph = take((size_t)pfc * m->Fl * 2);
-  const size_t o_pt = take((size_t)pfc * 4 + 4);
+  const bool pf_chosen = env_int("NFAI_PREFILL_CHUNK", 0) == env_int("NFAI_PREFILL_CHUNK", 1);  // (set from outside)
+  uint32_t pfc = want_pf ? std::min(hp.ctx, pf_want) : 0;
   // split-K happens only below 120 output tiles of 128 x 128, with at most one CTA per SM: that many tiles of partials bound it
   const size_t pf_part_floats = want_pf && env_int("NFAI_GEMM_SPLIT", 1) ? (size_t)sm_count() * 128 * 128 * 2 : 0;
-  const size_t o_pp = take(pf_part_floats * 4);
+  const size_t before_pf = arena.off;
+  size_t o_px0, o_px1, o_pa, o_pq, o_pao, o_ph, o_pt, o_pp;
+  cudaError_t e;
+  for (;;) {
+    o_px0 = take((size_t)pfc * hp.H * 4);
+    o_px1 = take((size_t)pfc * hp.H * 4);
+    o_pa = take((size_t)pfc * amax * 2);
+    o_pq = take((size_t)pfc * m->qDimL * 4);
+    o_pao = take((size_t)pfc * m->qDimL * 2);
+    o_ph = take((size_t)pfc * m->Fl * 2);
+    o_pt = take((size_t)pfc * 4 + 4);
+    o_pp = take(pf_part_floats * 4);
+    e = cudaMalloc((void**)&m->rarena, arena.off);
+    if (e == cudaSuccess || pf_chosen || pfc <= kShortPass) break;
+    cudaGetLastError();
+    arena.off = before_pf;
+    pfc = kShortPass;
+  }
   const size_t off = arena.off;
-  cudaError_t e = cudaMalloc((void**)&m->rarena, off);
   if (e != cudaSuccess) return fail(c, NFAI_ERR_OOM, "cudaMalloc of %zu run-time bytes (KV cache etc.): %s", off, cudaGetErrorString(e));
   CU(c, cudaMemsetAsync(m->rarena, 0, off, c->stream));
   m->kc = m->rarena + o_kc; m->vc = m->rarena + o_vc;
