@@ -80,7 +80,7 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 }
 // 2^x of a pair on the fused multiply-add units, for x below 128: x = n + f with n whole and |f| <= 1/2 (adding 1.5 * 2^23 rounds),
 // 2^f by its minimax polynomial of degree 5 (a linear program over the relative error; 2.1e-7 in float32, as much as the
-// hardware's approximation is allowed), n added to the exponent. Anything below 2^-126 becomes that; a NaN stays above all.
+// hardware's approximation is allowed), times 2^n (exact). Anything below 2^-126 becomes that; a NaN stays one.
 __device__ __forceinline__ void poly_ex2(uint64_t x2, float& a, float& b) {
   float x0, x1;
   unpair(x2, x0, x1);
@@ -97,8 +97,8 @@ __device__ __forceinline__ void poly_ex2(uint64_t x2, float& a, float& b) {
   float q0, q1, t0, t1;
   unpair(q, q0, q1);
   unpair(t, t0, t1);
-  a = __uint_as_float((__float_as_uint(t0) << 23) + __float_as_uint(q0));
-  b = __uint_as_float((__float_as_uint(t1) << 23) + __float_as_uint(q1));
+  a = q0 * __uint_as_float((__float_as_uint(t0) << 23) + 0x3f800000u);
+  b = q1 * __uint_as_float((__float_as_uint(t1) << 23) + 0x3f800000u);
 }
 
 template <int D>

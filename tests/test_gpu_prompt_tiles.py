@@ -97,6 +97,27 @@ def test_attention_tiles(factory, monkeypatch, heads, kv_heads, d, position, tok
         assert rel_err(a, b) < 2e-3  # (float32 sums in another order, rounded to float16 between the kernels: a few 2^-11)
 
 
+@pytest.mark.parametrize("at", [32, 33, 34, 300, 416])
+def test_a_key_that_is_not_a_number(factory, monkeypatch, at):
+    """Every exponential (positions 32, 33 and 416 go through the polynomial) passes a NaN on, as the warp-level kernel does."""
+    cfg = synth.get_config("s3", gain_std=0.1)
+    m = create_synthetic_model(cfg, 640, factory=factory, kv_dtype="f16")
+    rng = np.random.default_rng(at)
+    k, v = (rng.standard_normal((600, cfg.kvDim), dtype=np.float32) for _ in "kv")
+    k[at, :cfg.d] = np.nan
+    m.write_kv_range(0, 0, k, v)
+    ids = synth.prompt_ids(cfg, 33, 8)
+    out = {}
+    for kind in ("1", "2"):
+        monkeypatch.setenv("NFAI_PREFILL_ATTN", kind)
+        m.set_position(500)
+        m.prefill(ids)
+        out[kind] = [m.read_hidden(1)] + [a for p in (500, 532) for a in m.read_kv(1, p)]
+    m.Dispose()
+    for a, b in zip(out["1"], out["2"]):
+        assert np.isnan(a).all() and np.isnan(b).all()
+
+
 @pytest.mark.parametrize("key,tokens", [("s1", 1601), ("s2", 300), ("s1", 37)])
 def test_repeated_prompts_agree_to_the_bit(factory, key, tokens):
     """Kernels of every kind right behind one another (the next one's set-up runs beside the last one's end): what one leaves in
