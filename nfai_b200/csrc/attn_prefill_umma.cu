@@ -384,8 +384,10 @@ __global__ void __launch_bounds__(kUThreads, 2) attn_prefill_umma_kernel(const _
 template <int D>
 cudaError_t launch_umma(cudaStream_t s, const AttnParams& p, uint32_t T, uint32_t* err) {
   CUtensorMap mapK, mapV;
-  const uint64_t rows = (uint64_t)p.seq_imm - 1 + T, width = (uint64_t)p.kvH * D;  // (rows beyond the chunk come as zeros)
-  if (!tile_map16(&mapK, p.kcache, rows, width, kUN) || !tile_map16(&mapV, p.vcache, rows, width, kUN)) return cudaErrorInvalidValue;
+  // Rows beyond the chunk come as zeros, so a map is one pass's own: it is not kept (two per layer and pass would in time push
+  // those of the weights out).
+  const uint64_t rows = (uint64_t)p.seq_imm - 1 + T, width = (uint64_t)p.kvH * D;
+  if (!encode_tile_map16(&mapK, p.kcache, rows, width, kUN) || !encode_tile_map16(&mapV, p.vcache, rows, width, kUN)) return cudaErrorInvalidValue;
   static thread_local int attr_device = -1;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);

@@ -723,8 +723,9 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// A descriptor depends only on (address, rows, K, box rows); a prompt re-uses the same few hundred of them for every
-// chunk, so they are kept per host thread instead of being encoded again at each of ~130 launches per chunk.
+// A descriptor depends only on (address, rows, K, box rows). Those of the weights, the same few hundred for every pass, are kept per
+// host thread instead of being encoded again at each of ~110 launches, and with them those of the workspaces, a few per length of a
+// pass.
 struct MapKey {
   const void* base;
   uint64_t rows, K;
@@ -739,6 +740,17 @@ struct MapKeyHash {
 
 }  // namespace
 
+bool encode_tile_map16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32_t box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[2] = {K, rows};
+  cuuint64_t strides[1] = {K * 2};
+  cuuint32_t box[2] = {(cuuint32_t)kBK, box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool tile_map16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32_t box_rows) {
   static thread_local std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
   const MapKey key{base, rows, K, box_rows};
@@ -747,15 +759,7 @@ bool tile_map16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, u
     *map = it->second;
     return true;
   }
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  cuuint64_t dims[2] = {K, rows};
-  cuuint64_t strides[1] = {K * 2};
-  cuuint32_t box[2] = {(cuuint32_t)kBK, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  if (fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return false;
+  if (!encode_tile_map16(map, base, rows, K, box_rows)) return false;
   if (cache.size() > 4096) cache.clear();
   cache.emplace(key, *map);
   return true;

@@ -8,6 +8,8 @@
 namespace nfai {
 
 // Tensor map of [rows][K] 16-bit elements, K contiguous; box = 64 elements x box_rows rows, 128-byte swizzle, zero fill outside.
+bool encode_tile_map16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32_t box_rows);
+// The same, kept for the next call with the same arguments: for operands that come again.
 bool tile_map16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32_t box_rows);
 
 namespace umma {
