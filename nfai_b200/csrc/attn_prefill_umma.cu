@@ -37,6 +37,9 @@ constexpr uint32_t kUN = 128;        // positions per tile
 constexpr int kUThreads = 320;
 constexpr float kGrowth = 8.0f;      // growth of a maximum (base 2) that the sums are carried through without rescaling
 
+// A row's sum, or a NaN where it is beyond any sum of weights (2^kGrowth each): one of the scores was not a number
+__device__ __forceinline__ float known_sum(float l) { return l < 1e30f ? l : __uint_as_float(0x7fffffffu); }
+
 // Pairs of every eight whose exponentials go to the multiply-add units instead of the special function unit. Measured at 2048
 // tokens behind 28000 (d = 64, 32 heads): 0: 774 us, 1: 742, 2: 749, 3: 806, 4: 861; d = 128, 1024 behind 1024: 49.0, 48.8, 48.5,
 // 50.0, 51.9 us: the issue slots that the polynomial takes soon cost more than the special function unit is relieved of.
@@ -80,7 +83,9 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 }
 // 2^x of a pair on the fused multiply-add units, for x below 128: x = n + f with n whole and |f| <= 1/2 (adding 1.5 * 2^23 rounds),
 // 2^f by its minimax polynomial of degree 5 (a linear program over the relative error; 2.1e-7 in float32, as much as the
-// hardware's approximation is allowed), times 2^n (exact). Anything below 2^-126 becomes that; a NaN stays one.
+// hardware's approximation is allowed), n added to the exponent. Anything below 2^-126 becomes that; a NaN becomes the largest
+// finite number, which shows in the row's sum (known_sum; multiplying 2^n on would keep it one, but took 2392 us for 2378 at 9472 tokens
+// behind 18944, 47.0 for 46.2 at 2011 tokens of 24 heads of 128, looking at each tile's sum as much; this takes nothing).
 __device__ __forceinline__ void poly_ex2(uint64_t x2, float& a, float& b) {
   float x0, x1;
   unpair(x2, x0, x1);
@@ -97,8 +102,8 @@ __device__ __forceinline__ void poly_ex2(uint64_t x2, float& a, float& b) {
   float q0, q1, t0, t1;
   unpair(q, q0, q1);
   unpair(t, t0, t1);
-  a = q0 * __uint_as_float((__float_as_uint(t0) << 23) + 0x3f800000u);
-  b = q1 * __uint_as_float((__float_as_uint(t1) << 23) + 0x3f800000u);
+  a = __uint_as_float((__float_as_uint(t0) << 23) + __float_as_uint(q0));
+  b = __uint_as_float((__float_as_uint(t1) << 23) + __float_as_uint(q1));
 }
 
 template <int D>
@@ -287,7 +292,7 @@ __global__ void __launch_bounds__(kUThreads, 2) attn_prefill_umma_kernel(const _
             if (kAhead) ok = __all_sync(0xffffffffu, ok && bar_wait(pv_done, (it - 1) & 1));  // the sums of the tile before
             fence_after();
             const float f = u_ex2(m - top);
-            l *= f;
+            l = known_sum(l) * f;
 #pragma unroll 1
             for (uint32_t c = half * (D / 2); c < (half + 1) * (D / 2); c += 16) {
               uint32_t o[16];
@@ -351,11 +356,12 @@ __global__ void __launch_bounds__(kUThreads, 2) attn_prefill_umma_kernel(const _
     if (ok) ok = __all_sync(0xffffffffu, bar_wait(pv_done, (n - 1) & 1));
     if (ok) {
       fence_after();
-      const float inv = 1.0f / l;
+      const float inv = 1.0f / known_sum(l);
       __half* const out = p.out_half + (size_t)token * qDim + (size_t)(g * G + row % G) * D;
 #pragma unroll 1
       for (uint32_t c = half * (D / 2); c < (half + 1) * (D / 2); c += 32) {
         uint32_t o[32];
+
         tmem_ld(lanes + kO + c, o);
         if (token >= T) continue;
 #pragma unroll
