@@ -37,8 +37,9 @@ constexpr uint32_t kUN = 128;        // positions per tile
 constexpr int kUThreads = 320;
 constexpr float kGrowth = 8.0f;      // growth of a maximum (base 2) that the sums are carried through without rescaling
 
-// A row's sum, or a NaN where it is beyond any sum of weights (2^kGrowth each): one of the scores was not a number
-__device__ __forceinline__ float known_sum(float l) { return l < 1e30f ? l : __uint_as_float(0x7fffffffu); }
+// A row's sum, or a NaN where no weights add up to it: beyond any sum of them (2^kGrowth each) one of the scores was not a number;
+// below `least` (the whole row's has the 1 of its maximum) all were -infinity, and only the polynomial's 2^-126 are in it.
+__device__ __forceinline__ float known_sum(float l, float least) { return l >= least && l < 1e30f ? l : __uint_as_float(0x7fffffffu); }
 
 // Pairs of every eight whose exponentials go to the multiply-add units instead of the special function unit. Measured at 2048
 // tokens behind 28000 (d = 64, 32 heads): 0: 774 us, 1: 742, 2: 749, 3: 806, 4: 861; d = 128, 1024 behind 1024: 49.0, 48.8, 48.5,
@@ -292,7 +293,7 @@ __global__ void __launch_bounds__(kUThreads, 2) attn_prefill_umma_kernel(const _
             if (kAhead) ok = __all_sync(0xffffffffu, ok && bar_wait(pv_done, (it - 1) & 1));  // the sums of the tile before
             fence_after();
             const float f = u_ex2(m - top);
-            l = known_sum(l) * f;
+            l = known_sum(l, 0.f) * f;
 #pragma unroll 1
             for (uint32_t c = half * (D / 2); c < (half + 1) * (D / 2); c += 16) {
               uint32_t o[16];
@@ -356,12 +357,11 @@ __global__ void __launch_bounds__(kUThreads, 2) attn_prefill_umma_kernel(const _
     if (ok) ok = __all_sync(0xffffffffu, bar_wait(pv_done, (n - 1) & 1));
     if (ok) {
       fence_after();
-      const float inv = 1.0f / known_sum(l);
+      const float inv = 1.0f / known_sum(l, 0.5f);
       __half* const out = p.out_half + (size_t)token * qDim + (size_t)(g * G + row % G) * D;
 #pragma unroll 1
       for (uint32_t c = half * (D / 2); c < (half + 1) * (D / 2); c += 32) {
         uint32_t o[32];
-
         tmem_ld(lanes + kO + c, o);
         if (token >= T) continue;
 #pragma unroll
