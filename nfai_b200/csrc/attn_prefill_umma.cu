@@ -410,10 +410,19 @@ cudaError_t launch_umma(cudaStream_t s, const AttnParams& p, uint32_t T, uint32_
 
 }  // namespace
 
-// Up to 256 positions a walk is one or two tiles and the set-up of tensor memory and barriers is what counts: 128 tokens (32 heads
-// of 64) 5.2 us in the warp-level kernel, 6.4 here; 300 tokens, 6 heads: 8.7 and 8.7; 37 behind 603, 32 heads: 14.1 and 11.1.
+// The line to the warp-level kernel. A short walk is a few tiles, and the set-up of tensor memory and barriers counts as much:
+// with few rows (tokens times heads) up to 320 positions belong to the warp-level kernel (us, there and here: 64 tokens, 32 heads of
+// 64: 313 positions 8.9 and 9.4, 321: 9.4 and 8.9; 37 tokens, 24 heads of 128: 307: 11.5 and 13.1, 321: 13.0 and 13.2, 449: 16.7 and
+// 14.9; 37 of 32 heads of 64 at 640: 14.1 and 11.2). From 6144 rows on, heads of 64 fill that kernel's SMs more than once: 192
+// tokens of 32 heads at 257: 11.6 and 9.5 (160 tokens at 289: 9.4 and 10.1). Heads of 128 have one CTA of it on an SM and a tile of
+// 128 positions here costs them most where there are many: 300 tokens of 24 heads at 321: 13.3 and 14.8, 384 at 448: 16.5 and 17.1,
+// 449: 18.1 and 17.2.
 bool attn_prefill_umma_supported(int kvdtype, const AttnParams& p, uint32_t T) {
-  return kvdtype == 1 && (uint64_t)p.seq_imm - 1 + T > 256 && (p.d == 64 || p.d == 128) && (((uintptr_t)p.kcache | (uintptr_t)p.vcache | (uintptr_t)p.q | (uintptr_t)p.out_half) & 15) == 0;
+  if (kvdtype != 1 || (p.d != 64 && p.d != 128)) return false;
+  if ((((uintptr_t)p.kcache | (uintptr_t)p.vcache | (uintptr_t)p.q | (uintptr_t)p.out_half) & 15) != 0) return false;
+  const uint64_t rows = (uint64_t)T * p.qH;
+  const uint32_t short_walk = p.d == 64 ? (rows < 6144 ? 320 : 256) : (rows <= 4096 ? 320 : 448);
+  return (uint64_t)p.seq_imm - 1 + T > short_walk;
 }
 
 cudaError_t launch_attn_prefill_umma(cudaStream_t s, const AttnParams& p, uint32_t T, uint32_t* err) {

@@ -68,8 +68,9 @@ def factory():
     f.Dispose()
 
 
-@pytest.mark.parametrize("position,tokens", [(0, 257),     # the shortest walk taken: a third tile of one position
+@pytest.mark.parametrize("position,tokens", [(0, 257),     # a third tile of one position (the warp-level kernel's at these widths)
                                              (248, 9),     # the fewest tokens, rows of one CTA only in part
+                                             (0, 321), (312, 9),  # the same on the tcgen05 kernel
                                              (255, 130),
                                              (383, 33),    # the last position of a tile is the first token's own
                                              (1000, 517)])
@@ -95,6 +96,27 @@ def test_attention_tiles(factory, monkeypatch, heads, kv_heads, d, position, tok
     for a, b in zip(out["1"], out["2"]):
         assert np.isfinite(a).all()
         assert rel_err(a, b) < 2e-3  # (float32 sums in another order, rounded to float16 between the kernels: a few 2^-11)
+
+
+@pytest.mark.parametrize("heads,kv_heads,d,tokens,longest", [(8, 2, 64, 40, 320), (32, 8, 64, 191, 320), (32, 8, 64, 192, 256),
+                                                             (8, 8, 128, 300, 320), (24, 8, 128, 170, 320), (24, 8, 128, 171, 448)])
+def test_which_attention_runs(factory, monkeypatch, heads, kv_heads, d, tokens, longest):
+    """On either side of the line to the warp-level kernel: the same bits as that kernel's up to it, others (and close) beyond."""
+    cfg = synth.get_config("s3", qH=heads, kvH=kv_heads, d=d, gain_std=0.1)
+    m = create_synthetic_model(cfg, 512, factory=factory, kv_dtype="f16")
+    rng = np.random.default_rng(heads + tokens)
+    ids = synth.prompt_ids(cfg, tokens, 9)
+    for positions in (longest, longest + 1):
+        for layer in range(cfg.L):
+            m.write_kv_range(layer, 0, *(rng.standard_normal((512, cfg.kvDim), dtype=np.float32) for _ in "kv"))
+        out = {}
+        for kind in ("1", "2"):
+            monkeypatch.setenv("NFAI_PREFILL_ATTN", kind)
+            m.set_position(positions - tokens)
+            out[kind] = [m.prefill(ids)[0], m.read_hidden(0), m.read_hidden(1), *m.read_kv(1, positions - 1)]
+        assert all(np.array_equal(a, b) for a, b in zip(out["1"], out["2"])) == (positions <= longest)
+        assert all(rel_err(a, b) < 2e-3 for a, b in zip(out["1"], out["2"]))
+    m.Dispose()
 
 
 @pytest.mark.parametrize("at", [32, 33, 34, 300, 416])
