@@ -17,7 +17,7 @@ __device__ __forceinline__ void store_operand(const GemmEpilogue& ep, size_t at,
 // pair. The callers fetch it for a whole block of pairs before they touch the accumulators: a loop of load -> add ->
 // store per pair runs at one memory round trip per pair (the store may alias the next load as far as the compiler
 // knows), which cost more than the tile's MMAs.
-// KIND >= 0 fixes the epilogue at compile time (the persistent kernel dispatches once per tile); -1 reads ep.kind.
+// KIND >= 0 fixes the epilogue at compile time (the tensor-core kernels have an instance per kind); -1 reads ep.kind.
 template <int KIND = -1>
 __device__ __forceinline__ float2 epilogue_aux(const GemmEpilogue& ep, uint32_t m, uint32_t n, uint32_t N) {
   switch (KIND >= 0 ? KIND : (int)ep.kind) {

@@ -7,15 +7,18 @@
 // residual add) applied row by row.
 //
 // Shape of one CTA (320 threads, one 128 x BN output tile):
-//   warp 0      producer: one lane issues TMA tile loads (A 128x64, W BNx64 halves, 128-byte swizzle) into a ring of
-//               shared-memory stages, completion counted on the stage's "full" mbarrier;
-//   warp 1      MMA: allocates BN tensor-memory columns; one lane waits for a full stage, issues four
-//               tcgen05.mma (K = 16 each) from shared-memory descriptors, and commits to the stage's "empty"
-//               mbarrier so that the producer may refill it; after the last stage it commits to "accumulator ready";
+//   warp 0      producer: the warp waits for a free stage, an elected lane issues the TMA tile loads (A 128x64, W BNx64
+//               halves, 128-byte swizzle), completion counted on the stage's "full" mbarrier; at the end the warp waits
+//               for the last stages to be free again;
+//   warp 1      MMA: allocates BN tensor-memory columns; the warp waits for a full stage, an elected lane issues four
+//               tcgen05.mma (K = 16 each) from shared-memory descriptors and commits to the stage's "empty" mbarrier so
+//               that the producer may refill it, after the last stage also to "accumulator ready";
 //   warps 2-9   epilogue: two for each quarter of the accumulator's rows (a warp may only read the lanes of its index modulo 4),
 //               taking its column blocks in turn.
-// Larger products: pairs of CTAs (below). No tile copy is delivered to more than one CTA. Every mbarrier wait is bounded (one second): on a time-out the role
-// records an error bit and leaves; the tensor memory is released on every path.
+// K is split over several CTAs where the tiles alone leave SMs idle: they are a cluster and add up through each other's shared
+// memory, or, where too few clusters run at once, through memory and a second kernel. Larger products go to pairs of CTAs, rows
+// in groups to 128 x 256 tiles (both below). No tile copy is delivered to more than one CTA. Every mbarrier wait is bounded (one
+// second): on a time-out the role records an error bit and leaves; the tensor memory is released on every path.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -880,9 +883,10 @@ cudaError_t launch_grouped(cudaStream_t s, const __half* A, const __half* W, uin
 }
 
 // Columns of a pair's tile: the width in steps of 32 that needs the least time in waves of pairs (a wave costs its width, and
-// about 8 columns' worth of filling and draining), the wider one of two equal ones. 2011 x 3072 x 8192, forced: 256: 94.1 us,
-// 192 (the choice): 94.9, 160: 129, 128: 128; 2011 x 3072 x 2048: 34.6, 32.0, 41.3, 40.4; 2011 x 16384 x 2048: 116 at 256 (the
-// choice), 123 at 224, 132 at 192.
+// about 8 columns' worth of filling and draining), the wider one of two equal ones. Forced, with a residual and plain stores (us):
+// 2011 x 3072 x 8192: 256: 90, 224: 87, 192 (the choice): 81, 160: 100, 128: 103; 2011 x 3072 x 2048: 33, 31, 28, 33, 30;
+// 2011 x 16384 x 2048: 128 at 256 (the choice), 133 at 224, 137 at 192; 128 x 28672 x 4096: 63 at 256, 57 at 224 (the choice),
+// 71 at 192.
 uint32_t pair_columns(uint32_t M, uint32_t N) {
   const uint32_t pairs = sm_count() / 2, mt = (M + 2 * kBM - 1) / (2 * kBM);
   uint32_t best = 256, cost = ~0u;

@@ -28,8 +28,10 @@ struct GemmEpilogue {
   uint32_t qDim = 0, kvDim = 0, d = 0, ropeDim = 0, pos0 = 0;
   const float2* rope_cs = nullptr;
   // Optional scratch for split-K: when the tile grid alone would leave most SMs idle (a short prompt chunk), the K
-  // range is divided over several CTAs, each stores its float32 partial tile here ([split][M][N]) and a second
-  // kernel adds the partials in split order and applies the epilogue. Without scratch the GEMM never splits.
+  // range is divided over several CTAs. Where they fit into clusters, those add up their float32 sums in split order among
+  // themselves and the scratch is not touched; otherwise each stores its partial tile here ([split][M][N]) and a second
+  // kernel adds the partials in the same order and applies the epilogue. Without scratch the GEMM never splits, and never
+  // into more parts than the scratch holds: the caller chooses.
   float* scratch = nullptr;
   size_t scratch_floats = 0;
 };

@@ -26,7 +26,7 @@ def test_gemm_f16(cuda_ctx, M, N, K):
 
 
 def test_split_k_equals_single_pass(cuda_ctx, monkeypatch):
-    """A short chunk splits K over the SMs and adds the partial tiles in a second kernel: same product."""
+    """A short chunk splits K over the SMs, for this shape over clusters that add up among themselves: same product."""
     M, N, K = 128, 3072, 2048
     rng = np.random.default_rng(9)
     A = (rng.standard_normal((M, K)) * 0.5).astype(np.float16)
