@@ -3,7 +3,8 @@ tensor memory against the warp-level kernel of the same arithmetic."""
 import numpy as np
 import pytest
 
-from nfai_b200 import create_synthetic_model, LlamaModelFactory, synth
+from nfai_b200 import create_synthetic_model, LlamaModel, LlamaModelFactory, synth
+from nfai_b200.api import synthetic_tensors
 
 from .gpu_util import call, host, ptr, rel_err
 
@@ -138,6 +139,35 @@ def test_a_key_that_is_not_a_number(factory, monkeypatch, at):
     m.Dispose()
     for a, b in zip(out["1"], out["2"]):
         assert np.isnan(a).all() and np.isnan(b).all()
+
+
+def test_keys_beyond_float16(factory, monkeypatch):
+    """Every key's last component is -infinity in the cache and every query's is positive: all scores of a row are -infinity, and 0 / 0
+    is not a number in either kernel."""
+    cfg = synth.get_config("s3")
+    plain = synth.gen_tensor
+
+    def gen_tensor(cfg, name, *args):
+        w = plain(cfg, name, *args)
+        if name == "token_embd.weight":
+            w[:, 0] = 5.0  # (22 after the norm)
+        if name in ("blk.0.attn_q.weight", "blk.0.attn_k.weight"):
+            rows = [63] if "_k" in name else [63, 127, 191, 255]  # of the first KV group
+            w[rows] = 0
+            w[rows, 0] = -60000.0 if "_k" in name else 1.0
+        return w
+    monkeypatch.setattr(synth, "gen_tensor", gen_tensor)
+    metadata = dict(synth.metadata(cfg), **{"llama.rope.dimension_count": 32})  # (the last components are not rotated)
+    m = LlamaModel(factory.ctx, metadata, synthetic_tensors(cfg), 512, kv_dtype="f16")
+    ids = synth.prompt_ids(cfg, 400, 10)
+    for kind in ("1", "2"):
+        monkeypatch.setenv("NFAI_PREFILL_ATTN", kind)
+        m.reset()
+        m.prefill(ids)
+        k, _ = m.read_kv(0, 399)
+        assert k[63] == -np.inf and np.isfinite(np.delete(k, 63)).all()
+        assert np.isnan(m.read_hidden(0)).all(), kind
+    m.Dispose()
 
 
 @pytest.mark.parametrize("key,tokens", [("s1", 1601), ("s2", 300), ("s1", 37)])
