@@ -349,7 +349,7 @@ def run_ours(args, cfg):
                   "frac_of_sustained_bf16": flops / tsec / 1e12 / sus, "frac_of_burst_bf16": flops / tsec / 1e12 / burst,
                   "peak_kind": kind, "timing": "host clock around nfai_prefill with a synchronise on both sides, median of 5",
                   "flops": "2 x layer matrix params x T + causal attention 2 T^2 qDim L + one LM-head row"}
-    launches = model.step_launches()
+    launches = model.step_kernels()
     kv_bytes = 2 if model.kv_dtype == "f16" else 4
     first_pos = PROMPT_LEN + W
     step_bytes = sum(synth.decode_bytes(cfg, p, kv_bytes) for p in range(first_pos, first_pos + K)) / K / world

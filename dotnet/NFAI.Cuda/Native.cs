@@ -74,6 +74,7 @@ internal static unsafe partial class Native
     [DllImport(Lib)] internal static extern int nfai_op_attn_decode_static(IntPtr ctx, float* q, void* kcache, void* vcache, int kvDType, uint seq, uint qH, uint kvH, uint d, float* outp);
     [DllImport(Lib)] internal static extern int nfai_profile_kernel(IntPtr model, int which, int iters, out float avgMs, out ulong bytesPerLaunch);
     [DllImport(Lib)] internal static extern int nfai_step_launches(IntPtr model, out int launches);
+    [DllImport(Lib)] internal static extern int nfai_step_kernels(IntPtr model, out int kernels);
 
     internal static void Check(int status, IntPtr ctx)
     {

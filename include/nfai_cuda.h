@@ -284,8 +284,13 @@ int nfai_model_tune(nfai_model* m, int which, int mode, int rows_per_warp, int d
  * No counterpart in the reference. */
 int nfai_model_set_prefetch(nfai_model* m, uint64_t lookahead_bytes, uint64_t extra_bytes, int mode);
 
-/* Number of kernel launches inside one decode step (the captured graph's kernel nodes). */
+/* Number of kernel launches inside one decode step as a sequence of launches (the captured graph's kernel nodes): the kernels
+ * that nfai_profile_kernel times and nfai_model_tune shapes. */
 int nfai_step_launches(const nfai_model* m, int* out);
+
+/* Number of kernels that the step at the current position launches: 1 where the whole step is one resident kernel (float16
+ * models of some size on one GPU, caches of up to 4 096 positions, no launch shapes or look-ahead asked for), else as above. */
+int nfai_step_kernels(const nfai_model* m, int* out);
 
 /* ---- single kernels on caller-owned DEVICE buffers (kernel-level parity tests, embedding in other hosts) - */
 

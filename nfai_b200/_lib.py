@@ -95,6 +95,7 @@ SIGNATURES = {
     "nfai_model_tune": (_i, [_vp, _i, _i, _i, _i, _i]),
     "nfai_model_set_prefetch": (_i, [_vp, C.c_uint64, C.c_uint64, _i]),
     "nfai_step_launches": (_i, [_vp, C.POINTER(_i)]),
+    "nfai_step_kernels": (_i, [_vp, C.POINTER(_i)]),
     "nfai_op_embed": (_i, [_vp, _vp, _i, _u32, _u32, _u32, _vp]),
     "nfai_op_gemv": (_i, [_vp, _vp, _i, _u32, _u32, _vp, _vp, _f, _vp, _vp]),
     "nfai_op_qkv_rope": (_i, [_vp, _vp, _i, _vp, _vp, _f, _u32, _u32, _u32, _u32, _u32, _vp, _u32, _vp, _vp, _vp, _i]),

@@ -199,6 +199,11 @@ class CausalModel:
         check(self._lib.nfai_step_launches(self.handle, C.byref(n)), self.ctx.handle)
         return n.value
 
+    def step_kernels(self) -> int:
+        n = C.c_int()
+        check(self._lib.nfai_step_kernels(self.handle, C.byref(n)), self.ctx.handle)
+        return n.value
+
     def Dispose(self):
         if getattr(self, "handle", None):
             self._lib.nfai_model_destroy(self.handle)

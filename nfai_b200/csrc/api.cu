@@ -55,11 +55,12 @@ bool ring_wanted(uint32_t positions) {
 
 }  // namespace
 
-void nfai::read_tune(const char* name, GemvTune& t, int r_default, int u_default) {
+void nfai::read_tune(const char* name, GemvTune& t, int r_default, int u_default, bool* shaped) {
   t.rows_per_warp = r_default;
   t.unroll = u_default;
   std::string key = std::string("NFAI_TUNE_") + name;
   const char* v = getenv(key.c_str());
+  if (v && shaped) *shaped = true;
   if (v) {
     int r = 0, u = 0, cps = 0, mode = 0, split = 0, ahead = 0, grid = 0;
     int got = sscanf(v, "%d,%d,%d,%d,%d,%d,%d", &r, &u, &cps, &mode, &split, &ahead, &grid);
@@ -369,8 +370,59 @@ int capture(nfai_model* m, bool with_head, bool from_prompt, cudaGraphExec_t* ou
   return NFAI_OK;
 }
 
-int run_step(nfai_model* m, bool with_head, bool from_prompt) {
+// Whether the step runs as one resident kernel, and its layout. One GPU, caches of up to 4 096 positions (beyond, attention is most
+// of the step and runs on the tensor cores), and no launch shape asked for.
+bool plan_resident(nfai_model* m) {
   nfai_ctx* c = m->ctx;
+  const nfai_hparams& hp = m->hp;
+  if (c->world != 1 || !c->use_graph || m->shaped || hp.ctx > 4096 || m->attn_heads != 1) return false;
+  ResidentStep& p = m->step;
+  p.L = hp.L; p.H = hp.H; p.qH = hp.qH; p.kvH = hp.kvH; p.d = hp.d; p.F = hp.F; p.V = hp.V; p.ctx = hp.ctx; p.ropeDim = hp.ropeDim;
+  p.eps = hp.eps;
+  const LayerW& first = m->layers.front();
+  p.w[0] = first.qkv.ptr; p.w[1] = first.o.ptr; p.w[2] = first.gateup.ptr; p.w[3] = first.down.ptr;
+  p.w[4] = head_params(m).W;
+  p.attn_norm = first.attn_norm.ptr; p.ffn_norm = first.ffn_norm.ptr;
+  p.layer_stride = hp.L > 1 ? (uint64_t)((const char*)m->layers[1].qkv.ptr - (const char*)first.qkv.ptr) : 0;
+  for (uint32_t l = 0; l < hp.L; ++l) {  // layers lie in the arena one behind the other
+    const LayerW& w = m->layers[l];
+    const char* at[6] = {(const char*)w.qkv.ptr, (const char*)w.o.ptr, (const char*)w.gateup.ptr, (const char*)w.down.ptr, (const char*)w.attn_norm.ptr, (const char*)w.ffn_norm.ptr};
+    const char* base[6] = {(const char*)p.w[0], (const char*)p.w[1], (const char*)p.w[2], (const char*)p.w[3], (const char*)p.attn_norm, (const char*)p.ffn_norm};
+    for (int i = 0; i < 6; ++i)
+      if (at[i] != base[i] + l * p.layer_stride) return false;
+  }
+  p.embd = m->embd.ptr;
+  p.out_norm = m->out_norm.ptr;
+  return resident_plan(hp.weight_dtype, hp.kv_dtype, &p);
+}
+
+void bind_resident(nfai_model* m, char* words, char* counts) {
+  ResidentStep& p = m->step;
+  p.rope_cs = m->rope_cs;
+  p.state = m->state;
+  p.xbuf = m->xbuf;
+  p.kc = m->kc;
+  p.vc = m->vc;
+  p.logits = m->logits;
+  p.part_val = m->part_val;
+  p.part_idx = m->part_idx;
+  p.history = m->history;
+  p.history_cap = m->hp.ctx;
+  p.words = (unsigned long long*)words;
+  p.epoch = (uint32_t*)counts;
+  p.ticket = p.epoch + 1;
+}
+
+// The step at position `pos`: where the model stands when it runs.
+int run_step(nfai_model* m, bool with_head, bool from_prompt, uint32_t pos) {
+  nfai_ctx* c = m->ctx;
+  if (m->resident && pos < resident_positions(m->hp.d)) {
+    ResidentStep p = m->step;
+    p.with_head = with_head ? 1 : 0;
+    p.prompt = from_prompt ? m->prompt : nullptr;
+    CU(c, launch_step_resident(c->stream, m->hp.kv_dtype, p));
+    return NFAI_OK;
+  }
   if (c->use_graph) {
     CU(c, cudaGraphLaunch(with_head ? m->g_full : m->g_nohead, c->stream));
   } else {
@@ -757,11 +809,11 @@ int nfai_model_create(nfai_ctx* c, const nfai_hparams* hp, nfai_model** out) {
   m->pf_look = (uint64_t)env_int("NFAI_PF_MB", 0) << 20;
   m->pf_extra = (uint64_t)env_int("NFAI_PF_EXTRA_MB", 0) << 20;
   m->pf_mode = env_int("NFAI_PF_MODE", 1);
-  read_tune("QKV", m->tune_qkv, 2, 4);
-  read_tune("O", m->tune_o, 2, 4);
-  read_tune("GATEUP", m->tune_gateup, 2, 4);
-  read_tune("DOWN", m->tune_down, 2, 4);
-  read_tune("HEAD", m->tune_head, 2, 4);
+  read_tune("QKV", m->tune_qkv, 2, 4, &m->shaped);
+  read_tune("O", m->tune_o, 2, 4, &m->shaped);
+  read_tune("GATEUP", m->tune_gateup, 2, 4, &m->shaped);
+  read_tune("DOWN", m->tune_down, 2, 4, &m->shaped);
+  read_tune("HEAD", m->tune_head, 2, 4, &m->shaped);
   *out = m;
   return NFAI_OK;
 }
@@ -868,6 +920,9 @@ int nfai_model_finalize(nfai_model* m) {
   const size_t o_ap = take(attn_part_floats(m->qHl, hp.d, S_alloc) * 4);
   const size_t o_tk = take((size_t)m->qHl * 4);  // one ticket per (kv head, head group); at most one per query head
   const size_t o_tp = take((size_t)hp.H * 4);
+  m->resident = plan_resident(m);
+  const size_t o_words = take(m->resident ? (size_t)(hp.L + 1) * m->step.words_per_layer * 8 : 0);
+  const size_t o_counts = take(8);
   // batched prompt workspace
   const bool want_pf = hp.weight_dtype == NFAI_F16 && env_int("NFAI_PREFILL_GEMM", 1) != 0 &&
                        hp.H % 8 == 0 && m->qDimL % 8 == 0 && m->Fl % 8 == 0;
@@ -964,6 +1019,7 @@ int nfai_model_finalize(nfai_model* m) {
   }
   CU(c, cudaHostAlloc((void**)&m->pin_logits, (size_t)hp.V * 4, cudaHostAllocDefault));
   CU(c, cudaStreamSynchronize(c->stream));
+  if (m->resident) bind_resident(m, m->rarena + o_words, m->rarena + o_counts);
   int rc = capture_graphs(m);
   if (rc) return rc;
   m->pos = 0;
@@ -1011,7 +1067,7 @@ int nfai_decode(nfai_model* m, uint32_t token, float* logits, uint32_t* argmax) 
   if (m->pos >= m->hp.ctx) return fail(c, NFAI_ERR_CONTEXT_FULL, "position %u reached the KV-cache capacity %u", m->pos, m->hp.ctx);
   if (token >= m->hp.V) return fail(c, NFAI_ERR_ARG, "token id %u out of range (V = %u)", token, m->hp.V);
   if ((rc = set_state_word(m, offsetof(StepState, cur_token), token, 0))) return rc;
-  if ((rc = run_step(m, true, false))) return rc;
+  if ((rc = run_step(m, true, false, m->pos))) return rc;
   m->pos += 1;
   return fetch_outputs(m, logits, argmax);
 }
@@ -1131,10 +1187,10 @@ int nfai_prefill(nfai_model* m, const uint32_t* tokens, int n, float* logits_las
     CU(c, cudaMemcpyAsync(m->prompt, tokens, (size_t)(n - 1) * 4, cudaMemcpyHostToDevice, c->stream));
     if ((rc = set_state_word(m, offsetof(StepState, prompt_idx), 0, 1))) return rc;
     for (int i = 0; i < n - 1; ++i)
-      if ((rc = run_step(m, false, true))) return rc;
+      if ((rc = run_step(m, false, true, m->pos + (uint32_t)i))) return rc;
   }
   if ((rc = set_state_word(m, offsetof(StepState, cur_token), tokens[n - 1], 0))) return rc;
-  if ((rc = run_step(m, true, false))) return rc;
+  if ((rc = run_step(m, true, false, m->pos + (uint32_t)n - 1))) return rc;
   m->pos += (uint32_t)n;
   return fetch_outputs(m, logits_last, argmax_last);
 }
@@ -1178,7 +1234,7 @@ int nfai_decode_greedy(nfai_model* m, uint32_t first_token, int n_steps, uint32_
   if ((rc = set_state_word(m, offsetof(StepState, steps), 0, 2))) return rc;
   CU(c, cudaEventRecord(c->ev0, c->stream));
   for (int i = 0; i < n_steps; ++i)
-    if ((rc = run_step(m, true, false))) return rc;
+    if ((rc = run_step(m, true, false, m->pos + (uint32_t)i))) return rc;
   CU(c, cudaEventRecord(c->ev1, c->stream));
   m->pos += (uint32_t)n_steps;
   if ((rc = check_state(m, nullptr))) return rc;
@@ -1231,7 +1287,7 @@ int nfai_decode_sampled(nfai_model* m, uint32_t first_token, int n_steps, float 
   for (int i = 0; i < n_steps; ++i) {
     // the step leaves logits, arg-max and history[i] = arg-max; the sampler then puts the drawn token into history[i]
     // and into cur_token, which the next step embeds -- nothing returns to the host inside the loop
-    if ((rc = run_step(m, true, false))) return rc;
+    if ((rc = run_step(m, true, false, m->pos + (uint32_t)i))) return rc;
     CU(c, launch_sample_top_p(c->stream, m->logits, m->hp.V, &m->state->last_argmax, &m->state->cur_token, temperature, top_p,
                               top_k, u[i], m->sample_scratch, m->history + i));
   }
@@ -1467,6 +1523,7 @@ int nfai_model_tune(nfai_model* m, int which, int mode, int rows_per_warp, int d
   t->ctas_per_sm = ctas_per_sm;
   t->grid = grid;
   t->split = split;
+  m->shaped = true;
   if (!m->finalized) return NFAI_OK;
   CU(c, cudaSetDevice(c->device));
   CU(c, cudaStreamSynchronize(c->stream));
@@ -1481,6 +1538,7 @@ int nfai_model_tune(nfai_model* m, int which, int mode, int rows_per_warp, int d
   }
   int rc = capture_graphs(m);
   if (rc != NFAI_OK) *t = old;
+  else m->resident = false;
   return rc;
 }
 
@@ -1492,16 +1550,25 @@ int nfai_model_set_prefetch(nfai_model* m, uint64_t lookahead_bytes, uint64_t ex
   m->pf_look = lookahead_bytes;
   m->pf_extra = extra_bytes;
   m->pf_mode = mode;
+  m->shaped = true;
   if (!m->finalized || !c->use_graph) return NFAI_OK;
   CU(c, cudaSetDevice(c->device));
   CU(c, cudaStreamSynchronize(c->stream));
-  return capture_graphs(m);
+  int rc = capture_graphs(m);
+  if (rc == NFAI_OK) m->resident = false;
+  return rc;
 }
 
 int nfai_step_launches(const nfai_model* m, int* out) {
   if (!m || !out) return fail(m ? m->ctx : nullptr, NFAI_ERR_ARG, "null argument");
   *out = m->plan && !m->ctx->use_graph ? plan_step_launches(m) : m->launches_full;
   return NFAI_OK;
+}
+
+int nfai_step_kernels(const nfai_model* m, int* out) {
+  int rc = nfai_step_launches(m, out);
+  if (rc == NFAI_OK && m->resident && m->pos < resident_positions(m->hp.d)) *out = 1;
+  return rc;
 }
 
 int nfai_profile_kernel(nfai_model* m, int which, int iters, float* avg_ms, uint64_t* bytes_per_launch) {

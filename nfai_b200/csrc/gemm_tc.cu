@@ -754,6 +754,18 @@ bool encode_tile_map16(CUtensorMap* map, const void* base, uint64_t rows, uint64
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+bool encode_stack_map16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint64_t layers, uint64_t stride, uint32_t box_rows,
+                        uint32_t box_blocks) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn || K % kBK || stride % 16) return false;
+  cuuint64_t dims[4] = {kBK, rows, K / kBK, layers};
+  cuuint64_t strides[3] = {K * 2, kBK * 2, layers > 1 ? stride : rows * K * 2};
+  cuuint32_t box[4] = {(cuuint32_t)kBK, box_rows, box_blocks, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool tile_map16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32_t box_rows) {
   static thread_local std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
   const MapKey key{base, rows, K, box_rows};

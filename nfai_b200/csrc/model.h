@@ -12,6 +12,7 @@
 #include "../../include/nfai_cuda.h"
 #include "gemm_tc.h"
 #include "kernels.h"
+#include "step_resident.h"
 #include "tp.h"
 
 namespace nfai {
@@ -131,6 +132,9 @@ struct nfai_model {
   void* sample_scratch = nullptr;  // per-slice sums and candidates of the on-device sampler
   cudaGraphExec_t g_full = nullptr, g_nohead = nullptr;
   int launches_full = 0;
+  bool shaped = false;    // launch shapes or the L2 look-ahead were asked for: the step is the sequence of launches they belong to
+  bool resident = false;  // the step is one kernel (step_resident.cu)
+  ResidentStep step;
   uint32_t pos = 0;  // host mirror of state->pos
   GemvTune tune_qkv, tune_o, tune_gateup, tune_down, tune_head;
   // batched prompt path (float16 weights, one GPU): chunk workspace
@@ -174,7 +178,7 @@ int capture_graphs(nfai_model* m);
 int ready(nfai_model* m);
 int check_state(nfai_model* m, StepState* host_copy);
 int set_state_word(nfai_model* m, size_t offset, uint32_t value, int slot);
-void read_tune(const char* name, GemvTune& t, int r_default, int u_default);
+void read_tune(const char* name, GemvTune& t, int r_default, int u_default, bool* shaped = nullptr);  // *shaped: set from outside
 
 // ---- hooks of layer-plan models (plan_model.cu), called where the Llama path would run its own code --------------------------
 int plan_resolve(nfai_model* m, const char* name, const uint64_t* shape, int ndim, UploadTarget* t);

@@ -9,7 +9,11 @@ namespace nfai {
 
 // Tensor map of [rows][K] 16-bit elements, K contiguous; box = 64 elements x box_rows rows, 128-byte swizzle, zero fill outside.
 bool encode_tile_map16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32_t box_rows);
-// The same, kept for the next call with the same arguments: for operands that come again.
+// Tensor map of `layers` matrices of [rows][K] 16-bit elements, `stride` bytes apart (K a multiple of 64): box = 64 elements x box_rows
+// rows x box_blocks blocks of 64 elements, blocks outermost; 128-byte swizzle, zero fill outside. Coordinates: 0, row, block, layer.
+bool encode_stack_map16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint64_t layers, uint64_t stride, uint32_t box_rows,
+                        uint32_t box_blocks);
+// encode_tile_map16, kept for the next call with the same arguments: for operands that come again.
 bool tile_map16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32_t box_rows);
 
 namespace umma {

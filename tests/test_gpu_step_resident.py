@@ -1,0 +1,114 @@
+"""The decode step as one resident kernel, against a plain float64 statement and against the same step as a sequence of launches."""
+import numpy as np
+import pytest
+
+from nfai_b200 import LlamaModelFactory, create_synthetic_model, synth
+
+from .test_gpu_prompt_exact import PlainLlama, off
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module")
+def factory():
+    f = LlamaModelFactory(0)
+    yield f
+    f.Dispose()
+
+
+SHAPES = {
+    # x of 4 pieces, of 16 in four chunks; shares of 13 and 14 rows (boxes of 8, 4 and 2); an odd vocabulary
+    "heads of 64": dict(V=2053),
+    # 6 pieces; 2 816 columns: five pieces and a half; three query heads a KV head
+    "heads of 128": dict(H=3072, qH=24, kvH=8, d=128, F=2816, V=1111),
+    # 8 pieces, the most that are kept; one matrix of fewer columns than rows are dealt to
+    "eight pieces": dict(H=4096, qH=16, kvH=8, d=64, F=1536, V=777, tied=False),
+    # 3 pieces, one block of columns over 16 pieces; heads of 32 and eight of them a KV head
+    "heads of 32": dict(H=1536, qH=32, kvH=4, d=32, F=8256, V=512),
+}
+
+
+@pytest.mark.parametrize("shape,cache,position,ctx", [
+    ("heads of 64", "f32", 0, 64), ("heads of 64", "f16", 127, 256), ("heads of 64", "f32", 128, 256), ("heads of 64", "f16", 256, 1024),
+    ("heads of 64", "f16", 257, 4096), ("heads of 64", "f32", 4094, 4096), ("heads of 128", "f32", 1, 64), ("heads of 128", "f16", 128, 1024),
+    ("heads of 128", "f32", 1030, 2048), ("heads of 128", "f16", 3070, 4096), ("eight pieces", "f32", 63, 128), ("heads of 32", "f32", 300, 512),
+    ("heads of 32", "f16", 511, 1024)])
+def test_step(factory, shape, cache, position, ctx):
+    """Weights are multiplied exactly and summed in float32, as are scores and values: 2e-6 measured with float32 rows. The angles of
+    the rotation are products rounded to float32: off by up to position * 2^-24. The newest row of a float16 cache is rounded to
+    2^-11, of which a layer passes on less than it has."""
+    cfg = synth.get_config("s1", gain_std=0.1, **SHAPES[shape])
+    bound = 1e-5 + position * 2.0 ** -24 if cache == "f32" else 2e-3
+    rng = np.random.default_rng(position)
+    rows = [tuple(rng.standard_normal((position, cfg.kvDim)).astype(np.float16).astype(np.float32) for _ in "kv") for _ in range(cfg.L)]
+    m = create_synthetic_model(cfg, ctx, factory=factory, kv_dtype=cache)
+    assert m.step_kernels() == 1
+    if position:
+        for l in range(cfg.L):
+            m.write_kv_range(l, 0, *rows[l])
+        m.set_position(position)
+    assert (m.step_kernels() == 1) == (cfg.d < 128 or position < 3072)
+    plain, worst = PlainLlama(cfg), {}
+    for i, token in enumerate(synth.prompt_ids(cfg, 2, 5)):
+        new, streams, want = plain.prompt([token], rows)
+        got, best = m.decode(int(token))
+        worst[f"logits {i}"] = off(got, want)
+        assert best == int(np.argmax(got))
+        for l in range(cfg.L):
+            k, v = m.read_kv(l, position + i)
+            worst[f"rows {i} {l}"] = max(off(k, new[l][0][0]), off(v, new[l][1][0]))
+            worst[f"stream {i} {l}"] = off(m.read_hidden(l), streams[l])
+        rows = [tuple(np.concatenate((old, t.float().cpu().numpy())) for old, t in zip(rows[l], new[l])) for l in range(cfg.L)]
+    m.Dispose()
+    assert max(worst.values()) < bound, worst
+
+
+def test_loops_prompts_and_shapes(factory):
+    """Greedy loops repeat bit for bit, prompts too short for a pass go through steps without a head, and a model whose launch shapes
+    were asked for runs the launches they belong to."""
+    cfg = synth.get_config("s1", V=2053)
+    m = create_synthetic_model(cfg, 512, factory=factory)
+    ids = synth.prompt_ids(cfg, 5, 0)
+    runs = []
+    for _ in range(2):
+        m.reset()
+        first, best = m.prefill(ids)
+        tokens, _ = m.decode_greedy(best, 40)
+        last, _ = m.decode(tokens[-1])
+        runs.append((first.view(np.uint32).tolist(), list(tokens), last.view(np.uint32).tolist()))
+    assert runs[0] == runs[1]
+    m.reset()
+    for token in ids:
+        stepped, _ = m.decode(int(token))
+    assert np.array_equal(first.view(np.uint32), stepped.view(np.uint32))
+    m.tune("ffn_gate_up", 0, 2, 4, 2)
+    assert m.step_kernels() == m.step_launches()
+    m.reset()
+    again, best2 = m.prefill(ids)
+    # the cache is of float16: rows that lie between two of its numbers go either way
+    assert best2 == best and float(np.linalg.norm(again - first) / np.linalg.norm(first)) < 1e-3
+    m.Dispose()
+
+
+def test_extreme_inputs(factory):
+    """Rows that no float16 holds, and a layer that makes infinities: as the launches have them."""
+    cfg = synth.get_config("s1", V=2053)
+    logits = []
+    for shaped in (False, True):
+        m = create_synthetic_model(cfg, 64, factory=factory, kv_dtype="f32")
+        if shaped:
+            m.tune("ffn_gate_up", 0, 2, 4, 2)
+        rng = np.random.default_rng(0)
+        k, v = (rng.standard_normal((8, cfg.kvDim)).astype(np.float32) for _ in "kv")
+        for l in range(cfg.L):
+            m.write_kv_range(l, 0, k, v * (1e9 if l == 0 else 1e-9))
+        m.set_position(8)
+        large = m.decode(3)[0]
+        v[0, 0] = np.inf
+        m.write_kv_range(0, 0, k, v)
+        m.set_position(8)
+        logits.append((large, m.decode(3)[0]))
+        m.Dispose()
+    assert np.isfinite(logits[0][0]).all() and float(np.linalg.norm(logits[0][0] - logits[1][0]) / np.linalg.norm(logits[1][0])) < 1e-5
+    assert not np.isfinite(logits[0][1]).any() and not np.isfinite(logits[1][1]).any()
