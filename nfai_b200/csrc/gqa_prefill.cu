@@ -493,8 +493,9 @@ cudaError_t launch_gqa_prep(cudaStream_t s, const GqaParams& p, uint32_t T) {
 
 cudaError_t launch_gqa_prefill(cudaStream_t s, const GqaParams& p, uint32_t T) {
   if (!T || !p.in || !p.q || !p.ao || (uint64_t)p.pos0 + T > p.ctx) return cudaErrorInvalidValue;
-  static const bool tensor_cores = env_int("NFAI_PREFILL_ATTN", 1) != 0;
-  if (p.dtype == 2 && tensor_cores && mma_supported(p.spec)) {
+  const int kind = env_int("NFAI_PREFILL_ATTN", 1);
+  if (kind == 1 && gqa_prefill_umma_supported(p, T)) return launch_gqa_prefill_umma(s, p, T);
+  if (p.dtype == 2 && kind != 0 && mma_supported(p.spec)) {
     const uint32_t dim = p.spec.dim, dv = value_width(p.spec.vdim);
     if (dim > 32 && dim <= 64 && dv == 64) return launch_mma<64, 64, 64>(s, p, T);
     if (dim > 64 && dim <= 128 && dv == 128) return launch_mma<128, 128, 64>(s, p, T);

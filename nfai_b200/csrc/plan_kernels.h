@@ -147,7 +147,7 @@ struct GqaParams {
   void* v_cache = nullptr;     // [ctx][kv_heads*vdim] of dtype, normed
   int dtype = 0;               // of caches and operands: 0 or 2
   uint32_t ctx = 0;
-  StepState* state = nullptr;  // decode: position
+  StepState* state = nullptr;  // decode: position; prompt path: errors (may be null)
   uint32_t pos0 = 0;           // prompt path: position of the first token
   // decode
   float* out = nullptr;        // [heads*vdim], gated
@@ -164,6 +164,8 @@ cudaError_t launch_gqa_decode(cudaStream_t s, const GqaParams& p, bool pdl);
 // Norm what the projection of T tokens left: cache rows pos0 .. pos0+T-1 (unless borrowed) and p.q.
 cudaError_t launch_gqa_prep(cudaStream_t s, const GqaParams& p, uint32_t T);
 cudaError_t launch_gqa_prefill(cudaStream_t s, const GqaParams& p, uint32_t T);
+bool gqa_prefill_umma_supported(const GqaParams& p, uint32_t T);  // gqa_prefill_umma.cu
+cudaError_t launch_gqa_prefill_umma(cudaStream_t s, const GqaParams& p, uint32_t T);
 
 // ---- routed feed-forwards over rows of tokens (moe.cu) -------------------------------------------------------------------
 struct MoeRows {

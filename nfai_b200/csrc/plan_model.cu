@@ -978,6 +978,7 @@ cudaError_t mixer_pass(nfai_model* m, uint32_t l, uint32_t pos0, uint32_t T) {
     p.pos0 = pos0;
     p.q = P->pQ;
     p.ao = P->pA;
+    p.state = m->state;
     if ((e = launch_gqa_prep(s, p, T)) != cudaSuccess) return e;
     return launch_gqa_prefill(s, p, T);
   }

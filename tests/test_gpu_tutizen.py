@@ -171,6 +171,27 @@ def test_attention_alone(cuda_ctx, mixer, dtype):
     alone(cuda_ctx, cfg, U.weights(cfg, 11), toks, dtype)
 
 
+@pytest.mark.parametrize("portions", [(64,), (65, 64), (127, 128), (129, 66, 191), (320, 321)], ids=str)
+@pytest.mark.parametrize("mixer", [U.attn(6, 2, 64, 64), U.attn(8, 2, 64, 64, scale=0.02), U.attn(3, 1, 128, 128, scale=0.8)], ids=str)
+def test_prompt_attention_on_whole_tiles(cuda_ctx, mixer, portions, monkeypatch):
+    """Portions that begin and end at and beside the tiles' edges (64 positions, 128 tokens), heads that reach all of them and a few only:
+    against the plain statement, and against the warp-level kernel, from which only sums in another order and their roundings to
+    bfloat16 (2^-9 each) set it apart."""
+    cfg = U.config([U.layer(mixer), U.layer(dict(mixer, kv_from=0, scale=0.7 * mixer["scale"]))], 64, 96)
+    W = U.weights(cfg, 12)
+    toks = np.random.default_rng(sum(portions)).integers(0, 96, sum(portions)).tolist()
+    want = P.forward(cfg, to64(W), toks, cache=bf16)
+    m, got = build(cuda_ctx, cfg, W, "bf16", 700), {}
+    for kind in ("1", "2"):
+        monkeypatch.setenv("NFAI_PREFILL_ATTN", kind)
+        m.reset()
+        ends = np.cumsum(portions)
+        got[kind] = np.concatenate([m.forward(toks[e - n:e], range(n)) for n, e in zip(portions, ends)])
+        assert U.error(got[kind], want) < TOL["bf16"], kind
+    m.Dispose()
+    assert U.error(got["1"], got["2"]) < 8 * 2.0 ** -9
+
+
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 def test_feed_forward_alone(cuda_ctx, dtype):
     """The attention's output matrix is zero (its bias stays): what is left are clamped feed-forwards and the residual. Values
