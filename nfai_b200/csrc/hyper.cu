@@ -42,13 +42,13 @@ __device__ __forceinline__ void stv(float* p, const Vec<V>& v) {
 }
 
 // ST >= S streams held in registers; V elements per thread and step
-template <int ST, int V>
-__global__ void __launch_bounds__(256, ST <= 4 ? 3 : 1) hyper_rows_kernel(const HyperRows p) {
+template <int ST, int V, int TH>
+__global__ void __launch_bounds__(TH, ST <= 4 ? 1024 / TH : 1) hyper_rows_kernel(const HyperRows p) {
   extern __shared__ __align__(16) float hsm[];
   float* us = hsm;  // [H] combined row
-  __shared__ float w_mix[kMaxStreams * kMaxStreams], w_out[kMaxStreams], w_in[kMaxStreams], red[8];
+  __shared__ float w_mix[kMaxStreams * kMaxStreams], w_out[kMaxStreams], w_in[kMaxStreams], red[TH / 32];
   const uint32_t S = p.S, H = p.H, tid = threadIdx.x;
-  for (uint32_t i = tid; i < S * S; i += 256) w_mix[i] = p.mix ? p.mix[i] : 0.f;
+  for (uint32_t i = tid; i < S * S; i += TH) w_mix[i] = p.mix ? p.mix[i] : 0.f;
   if (tid < S) {
     w_out[tid] = p.out ? p.out[tid] : 0.f;
     w_in[tid] = p.next_in ? p.next_in[tid] : 1.f;
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(256, ST <= 4 ? 3 : 1) hyper_rows_kernel(const 
   const size_t erow = p.tokens ? (size_t)p.tokens[blockIdx.x] * H : 0;
   float ss = 0.f;
 #pragma unroll 1
-  for (uint32_t i = tid * V; i < H; i += 256 * V) {
+  for (uint32_t i = tid * V; i < H; i += TH * V) {
     Vec<V> x[ST];
     if (p.tokens) {
 #pragma unroll
@@ -76,34 +76,28 @@ __global__ void __launch_bounds__(256, ST <= 4 ? 3 : 1) hyper_rows_kernel(const 
       for (int s = 0; s < ST; ++s)
         if (s < (int)S) x[s] = ldv<V>(X + (size_t)s * H + i);
     }
-    if (p.y) {
-      const Vec<V> y = ldv<V>(p.y + row * H + i);
-      Vec<V> n[ST];
+    Vec<V> y, u;
+    if (p.y) y = ldv<V>(p.y + row * H + i);
 #pragma unroll
-      for (int t = 0; t < ST; ++t)
-        if (t < (int)S) {
+    for (int e = 0; e < V; ++e) u.f[e] = 0.f;
 #pragma unroll
-          for (int e = 0; e < V; ++e) n[t].f[e] = w_out[t] * y.f[e];
+    for (int t = 0; t < ST; ++t)
+      if (t < (int)S) {  // one stream at a time: four in quads leave room for 1024 threads on an SM
+        Vec<V> n = x[t];
+        if (p.y) {
+#pragma unroll
+          for (int e = 0; e < V; ++e) n.f[e] = w_out[t] * y.f[e];
 #pragma unroll
           for (int s = 0; s < ST; ++s)
             if (s < (int)S) {
               const float w = w_mix[s * S + t];
 #pragma unroll
-              for (int e = 0; e < V; ++e) n[t].f[e] = fmaf(w, x[s].f[e], n[t].f[e]);
+              for (int e = 0; e < V; ++e) n.f[e] = fmaf(w, x[s].f[e], n.f[e]);
             }
         }
+        if (Xo) stv<V>(Xo + (size_t)t * H + i, n);
 #pragma unroll
-      for (int t = 0; t < ST; ++t) x[t] = n[t];
-    }
-    Vec<V> u;
-#pragma unroll
-    for (int e = 0; e < V; ++e) u.f[e] = 0.f;
-#pragma unroll
-    for (int t = 0; t < ST; ++t)
-      if (t < (int)S) {
-        if (Xo) stv<V>(Xo + (size_t)t * H + i, x[t]);
-#pragma unroll
-        for (int e = 0; e < V; ++e) u.f[e] = fmaf(w_in[t], x[t].f[e], u.f[e]);
+        for (int e = 0; e < V; ++e) u.f[e] = fmaf(w_in[t], n.f[e], u.f[e]);
       }
     if (p.u_out) stv<V>(p.u_out + (size_t)blockIdx.x * H + i, u);
     stv<V>(us + i, u);
@@ -116,9 +110,9 @@ __global__ void __launch_bounds__(256, ST <= 4 ? 3 : 1) hyper_rows_kernel(const 
   __syncthreads();
   float tot = 0.f;
 #pragma unroll
-  for (int w = 0; w < 8; ++w) tot += red[w];
+  for (int w = 0; w < TH / 32; ++w) tot += red[w];
   const float rms = sqrtf(__fdiv_rn(tot, (float)H) + p.eps);
-  for (uint32_t i = tid * V; i < H; i += 256 * V) {
+  for (uint32_t i = tid * V; i < H; i += TH * V) {
     const Vec<V> u = ldv<V>(us + i), g = ldv<V>(p.gain + i);
     float o[V];
 #pragma unroll
@@ -138,15 +132,24 @@ template <int ST>
 cudaError_t launch_st(cudaStream_t s, const HyperRows& p, uint32_t n) {
   const size_t smem = (size_t)p.H * 4;
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
-  auto kern = hyper_rows_kernel<ST, 1>;
+  auto kern = hyper_rows_kernel<ST, 1, 256>;
+  unsigned threads = 256;
   if constexpr (ST <= 8) {  // more streams would not fit the register file in quads
-    if (p.H % 4 == 0) kern = hyper_rows_kernel<ST, 4>;
+    if (p.H % 4 == 0) kern = hyper_rows_kernel<ST, 4, 256>;
+  }
+  if constexpr (ST <= 4) {
+    // Rows wider than 256 quads: all of a row of 2048 is in flight at once, on 1024 threads of an SM (256 a CTA and 768: 35.0 us for
+    // the 159 MB of 2011 tokens of 4 streams, 512: 29.9, 5.3 TB/s).
+    if (p.H % 4 == 0 && p.H > 1024) {
+      kern = hyper_rows_kernel<ST, 4, 512>;
+      threads = 512;
+    }
   }
   if (smem > 40 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  return launch_pdl(kern, dim3(n), dim3(256), smem, s, prefill_pdl(), p);
+  return launch_pdl(kern, dim3(n), dim3(threads), smem, s, prefill_pdl(), p);
 }
 
 template <typename WT>
