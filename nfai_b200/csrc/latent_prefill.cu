@@ -232,13 +232,29 @@ __global__ void __launch_bounds__(W * 32, DV <= 128 ? 2 : 1) latent_prefill_mma_
     const float inv = 1.0f / (half ? l_b : l_a);
     const float* gate = p.in + (size_t)row * p.in_ld + s.q_rows() + s.kv_rows() + (size_t)h * vdim;
     __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.ao) + (size_t)row * s.gate_rows() + (size_t)h * vdim;
+    constexpr int kBatch = DV / 8 < 16 ? DV / 8 : 16;  // gates before the stores that may alias them
 #pragma unroll
-    for (int j = 0; j < DV / 8; ++j)
+    for (int j0 = 0; j0 < DV / 8; j0 += kBatch) {
+      float z[kBatch][2];
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const uint32_t c = j * 8 + qc + e;
-        if (c < vdim) store_as(out + c, o[j][half * 2 + e] * inv * (1.0f / (1.0f + expf(-gate[c]))));
+      for (int j = 0; j < kBatch; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const uint32_t c = (j0 + j) * 8 + qc + e;
+          z[j][e] = c < vdim ? gate[c] : 0.f;
+        }
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j) {
+        const uint32_t c = (j0 + j) * 8 + qc;
+        const float a = o[j0 + j][half * 2] * inv * (1.0f / (1.0f + expf(-z[j][0]))), b = o[j0 + j][half * 2 + 1] * inv * (1.0f / (1.0f + expf(-z[j][1])));
+        if (vec) {
+          if (c < vdim) *reinterpret_cast<uint32_t*>(out + c) = pack_bf(a, b);
+        } else {
+          if (c < vdim) store_as(out + c, a);
+          if (c + 1 < vdim) store_as(out + c + 1, b);
+        }
       }
+    }
   }
 }
 
