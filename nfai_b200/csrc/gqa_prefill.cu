@@ -11,7 +11,8 @@
 //                      nothing in its softmax, so the bias of a key is taken relative to the warp's first token: the part
 //                      inside a tile is what the score accumulators start from, the part of the tile itself goes into the
 //                      subtraction of the maximum. Scores, exponentials and sums are float32, the weights enter the second
-//                      product as a bfloat16 head and remainder (relative error ~2^-17).
+//                      product as a bfloat16 head and remainder (relative error ~2^-17). Heads of 64 and 128 go to
+//                      gqa_prefill_umma.cu from 64 tokens on.
 //   gqa_prefill_simt   the same for true float32 and for head sizes the former does not take.
 // A portion may start anywhere: earlier positions are read from the cache.
 #include <algorithm>
