@@ -41,12 +41,16 @@ __device__ __forceinline__ void stv(float* p, const Vec<V>& v) {
   else *p = v.f[0];
 }
 
+// Threads that a row's squares are added up over, whatever the CTA has: the order of the sum, and with it the last bit of a row's
+// root mean square, does not follow from how many threads the streams are read with.
+constexpr int kSumThreads = 256;
+
 // ST >= S streams held in registers; V elements per thread and step
 template <int ST, int V, int TH>
 __global__ void __launch_bounds__(TH, ST <= 4 ? 1024 / TH : 1) hyper_rows_kernel(const HyperRows p) {
   extern __shared__ __align__(16) float hsm[];
   float* us = hsm;  // [H] combined row
-  __shared__ float w_mix[kMaxStreams * kMaxStreams], w_out[kMaxStreams], w_in[kMaxStreams], red[TH / 32];
+  __shared__ float w_mix[kMaxStreams * kMaxStreams], w_out[kMaxStreams], w_in[kMaxStreams], red[kSumThreads / 32];
   const uint32_t S = p.S, H = p.H, tid = threadIdx.x;
   for (uint32_t i = tid; i < S * S; i += TH) w_mix[i] = p.mix ? p.mix[i] : 0.f;
   if (tid < S) {
@@ -101,16 +105,30 @@ __global__ void __launch_bounds__(TH, ST <= 4 ? 1024 / TH : 1) hyper_rows_kernel
       }
     if (p.u_out) stv<V>(p.u_out + (size_t)blockIdx.x * H + i, u);
     stv<V>(us + i, u);
+    if constexpr (TH == kSumThreads) {
 #pragma unroll
-    for (int e = 0; e < V; ++e) ss = fmaf(u.f[e], u.f[e], ss);
+      for (int e = 0; e < V; ++e) ss = fmaf(u.f[e], u.f[e], ss);
+    }
   }
   if (!p.normed) return;
-  ss = warp_sum(ss);
-  if ((tid & 31) == 0) red[tid >> 5] = ss;
+  if constexpr (TH != kSumThreads) {
+    __syncthreads();
+    if (tid < kSumThreads) {
+      for (uint32_t i = tid * V; i < H; i += kSumThreads * V) {
+        const Vec<V> u = ldv<V>(us + i);
+#pragma unroll
+        for (int e = 0; e < V; ++e) ss = fmaf(u.f[e], u.f[e], ss);
+      }
+    }
+  }
+  if (tid < kSumThreads) {
+    ss = warp_sum(ss);
+    if ((tid & 31) == 0) red[tid >> 5] = ss;
+  }
   __syncthreads();
   float tot = 0.f;
 #pragma unroll
-  for (int w = 0; w < TH / 32; ++w) tot += red[w];
+  for (int w = 0; w < kSumThreads / 32; ++w) tot += red[w];
   const float rms = sqrtf(__fdiv_rn(tot, (float)H) + p.eps);
   for (uint32_t i = tid * V; i < H; i += TH * V) {
     const Vec<V> u = ldv<V>(us + i), g = ldv<V>(p.gain + i);

@@ -177,6 +177,44 @@ def test_feed_forward_alone(cuda_ctx, dtype):
     alone(cuda_ctx, cfg, W, list(range(50)), dtype)
 
 
+@pytest.mark.parametrize("width", [1024, 1028, 2048, 3072, 4100])
+@pytest.mark.parametrize("streams", [1, 4])
+def test_a_rows_norm_does_not_depend_on_the_threads(cuda_ctx, streams, width):
+    """A row's squares are added by 256 threads, in quads, then over warps by halves, then warp by warp, at any width: what the
+    operands of all further products round to follows from it. Nothing is left of the sublayers here, and the output matrix is
+    the identity: logits are the normed rows, bit for bit."""
+    cfg = U.config([U.layer(U.ssm(1, 24, 8, 1, 1, 1))], width, width, streams)
+    W = U.weights(cfg, 4)
+    for name in W:
+        if name.endswith(".o"):
+            W[name] = np.zeros_like(W[name])
+        elif name.endswith("mix"):
+            W[name] = np.eye(streams, dtype=np.float32)
+    W["head"] = np.eye(width, dtype=np.float32)
+    m = build(cuda_ctx, cfg, W, "f32", 64)
+    toks = np.random.default_rng(width).integers(0, width, 24).tolist()
+    got = m.forward(toks, range(len(toks)))
+    m.Dispose()
+    f32, lanes = np.float32, np.arange(32)
+    u = f32(streams) * W["embed"][toks]  # (exact: the embedding is bfloat16)
+    quads = np.zeros((len(toks), -(-width // 1024), 256, 4), f32)
+    quads.reshape(len(toks), -1)[:, :width] = u
+    sums = np.zeros((len(toks), 256), f32)
+    for k in range(quads.shape[1]):
+        for e in range(4):
+            x = quads[:, k, :, e].astype(np.float64)
+            sums = (x * x + sums).astype(f32)
+    sums = sums.reshape(-1, 8, 32)
+    for o in (16, 8, 4, 2, 1):
+        sums = sums + sums[:, :, lanes ^ o]
+    total = np.zeros(len(toks), f32)
+    for w in range(8):
+        total = total + sums[:, w, 0]
+    rms = np.sqrt(total / f32(width) + f32(cfg["norm"]["eps"]))
+    want = (u / rms[:, None]) * W["final.norm"]
+    assert np.array_equal(got, want)
+
+
 @pytest.mark.parametrize("streams", [1, 2, 5, 8, 9, 16])
 def test_stream_counts(cuda_ctx, streams):
     cfg = U.config([U.layer(U.latent(2, 16, 8, 16, 24, 9), 40), U.layer(U.ssm(2, 16, 8, 1, 3, 2))], 48, 40, streams)
