@@ -24,6 +24,7 @@
 // Reference arithmetic replaced: AttentionScoreCalculationShader.cs:170-205, AttentionSoftmaxShader.cs:145-177,
 // AttentionWeightedValueSumShader.cs:181-215, applied once per prompt token by LlamaModel.cs:103-126.
 #include "attn_core.cuh"
+#include "attn_phases.h"
 #include "umma.cuh"
 
 namespace nfai {
@@ -36,6 +37,7 @@ constexpr uint32_t kUM = 128;        // rows (token, head of the group) per CTA
 constexpr uint32_t kUN = 128;        // positions per tile
 constexpr int kUThreads = 320;
 constexpr float kGrowth = 8.0f;      // growth of a maximum (base 2) that the sums are carried through without rescaling
+using Values = ValuePhases<1>;       // the barrier of the products with the values
 
 // A row's sum, or a NaN where no weights add up to it: beyond any sum of them (2^kGrowth each) one of the scores was not a number;
 // below `least` (the whole row's has the 1 of its maximum) all were -infinity, and only the polynomial's 2^-126 are in it.
@@ -261,9 +263,13 @@ __global__ void __launch_bounds__(kUThreads, 2) attn_prefill_umma_kernel(const _
           : "memory");
       return r != 0;
     };
+    auto value = [&](uint32_t j) {  // the product of tile j with its values is done
+      ok = __all_sync(0xffffffffu, ok && bar_wait(pv_done, Values::parity(j)));
+    };
     float m = 0.f, l = 0.f;
     for (uint32_t it = 0; it < n; ++it) {
       ok = __all_sync(0xffffffffu, ok && bar_wait(s_ready, it & 1));  // (a warp that gave up still meets the other one)
+      if (!kAhead) Values::at_tile(it, value);
       const uint32_t n0 = it * kUN + col0;
       // The weights are formed from the maximum as it stands; a row that turns out to have grown too far (the first tile always
       // has) makes its two warps raise their maxima and do the tile again.
@@ -290,7 +296,7 @@ __global__ void __launch_bounds__(kUThreads, 2) attn_prefill_umma_kernel(const _
           meet();
           top = fmaxf(fmaxf(top, swap[(half ^ 1) * kUM + r_own]), it ? m : attn_detail::kNegBig);
           if (it) {
-            if (kAhead) ok = __all_sync(0xffffffffu, ok && bar_wait(pv_done, (it - 1) & 1));  // the sums of the tile before
+            Values::at_rescaling(it, value);
             fence_after();
             const float f = u_ex2(m - top);
             l = known_sum(l, 0.f) * f;
@@ -335,7 +341,7 @@ __global__ void __launch_bounds__(kUThreads, 2) attn_prefill_umma_kernel(const _
           fence_before();
           __syncwarp();
           if (lane == 0) bar_arrive(s_free);
-          if (it) ok = __all_sync(0xffffffffu, ok && bar_wait(pv_done, (it - 1) & 1));  // the weights of the tile before have been used
+          Values::at_tile(it, value);  // the weights of the tile before have been used
           fence_after();
         }
         tmem_st(lanes + kP + col0 / 2, w[0]);
@@ -354,7 +360,7 @@ __global__ void __launch_bounds__(kUThreads, 2) attn_prefill_umma_kernel(const _
     swap[half * kUM + r_own] = l;
     meet();
     l += swap[(half ^ 1) * kUM + r_own];
-    if (ok) ok = __all_sync(0xffffffffu, bar_wait(pv_done, (n - 1) & 1));
+    Values::at_end(n, value);
     if (ok) {
       fence_after();
       const float inv = 1.0f / known_sum(l, 0.5f);

@@ -15,6 +15,7 @@
 // gqa_prefill.cu, prompts of 16 layers with 32 heads of 64 (ms): 2011 tokens 6.54 and 5.97 (about 75 and 39 us a layer), 1024: 4.00 and
 // 3.91, 512: 3.04 and 2.99, 384: 2.88 and 2.83. Tiles of 128 positions, their weights over the scores of the only tile that fits beside
 // O then: 6.18 at 2011 (spills, and the products wait for the weights and the weights for the products).
+#include "attn_phases.h"
 #include "gqa_common.cuh"
 #include "umma.cuh"
 
@@ -30,6 +31,7 @@ constexpr uint32_t kM = 128;        // tokens of a CTA
 constexpr uint32_t kN = 64;         // positions per tile
 constexpr int kThreads = 320;
 constexpr float kGrowth = 8.0f;     // growth of a maximum (base 2) that the sums are carried through without rescaling
+using Values = ValuePhases<2>;      // barriers of the products with the values: scores are multiplied one tile ahead of them
 
 template <int D>
 struct Smem {
@@ -71,9 +73,9 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_prefill_umma_kernel(const __g
   extern __shared__ unsigned char gu_raw[];
   unsigned char* const sm = reinterpret_cast<unsigned char*>(((uintptr_t)gu_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* const bars = reinterpret_cast<uint64_t*>(sm + SM::kBarOff);
-  uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * SM::kSlots + 6);
+  uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * SM::kSlots + 5 + Values::kBarriers);
   const uint32_t full0 = s_u32(bars), empty0 = s_u32(bars + SM::kSlots), q_ready = s_u32(bars + 2 * SM::kSlots), s_ready = q_ready + 8,
-                 p_ready = q_ready + 24, pv_done = q_ready + 40;  // (s_ready, p_ready: one for each of two tiles)
+                 p_ready = q_ready + 24, pv_done = q_ready + 40;  // (s_ready, p_ready, pv_done: one for each of two tiles)
   const GqaSpec& spec = p.spec;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  // (warp: uniform)
   if (tid == 0) {
@@ -86,7 +88,7 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_prefill_umma_kernel(const __g
       bar_init(s_ready + 8 * i, 1);
       bar_init(p_ready + 8 * i, 8);
     }
-    bar_init(pv_done, 1);
+    for (uint32_t i = 0; i < Values::kBarriers; ++i) bar_init(pv_done + 8 * i, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 9) {
@@ -183,7 +185,7 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_prefill_umma_kernel(const __g
           umma_f16_ta(tmem + kO, weights + kLow + kk * 8, v, idesc_o, 1);
         }
         umma_commit(empty0 + 8 * s);
-        umma_commit(pv_done);
+        umma_commit(pv_done + 8 * Values::barrier(it));
       }
       __syncwarp();
     }
@@ -203,9 +205,13 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_prefill_umma_kernel(const __g
           : "memory");
       return r != 0;
     };
+    auto value = [&](uint32_t j) {  // the product of tile j with its values is done
+      ok = __all_sync(0xffffffffu, ok && bar_wait(pv_done + 8 * Values::barrier(j), Values::parity(j)));
+    };
     float m = kNegBig, l = 0.f;
     for (uint32_t it = 0; it < n; ++it) {
       ok = __all_sync(0xffffffffu, ok && bar_wait(s_ready + 8 * (it & 1), (it >> 1) & 1));  // (a warp that gave up still meets the other one)
+      Values::at_tile(it, value);
       const uint32_t n0 = (tile_hi - it) * kN + col0;
       const uint32_t tile = lanes + (it & 1) * kN;
       const float base = sl * (float)((int)n0 - (int)limit);  // bias of this half's first position
@@ -236,7 +242,7 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_prefill_umma_kernel(const __g
           meet();
           top = fmaxf(fmaxf(top, swap[(half ^ 1) * kM + r_own]), m);
           if (it) {
-            ok = __all_sync(0xffffffffu, ok && bar_wait(pv_done, (it - 1) & 1));  // the sums of the tile before (those before it came before these scores)
+            Values::at_rescaling(it, value);
             fence_after();
             const float f = gqa_ex2(m - top);
             l *= f;
@@ -279,8 +285,6 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_prefill_umma_kernel(const __g
       float s0, s1;
       unpair(add2(sum[0], sum[1]), s0, s1);
       l += s0 + s1;
-      // the last wait below is for the phase that ends next: the one before has ended, and the last cannot before this warp arrives
-      if (it && it + 1 == n) ok = __all_sync(0xffffffffu, ok && bar_wait(pv_done, (it - 1) & 1));
       tmem_st_wait();
       fence_before();
       __syncwarp();
@@ -289,7 +293,7 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_prefill_umma_kernel(const __g
     swap[half * kM + r_own] = l;
     meet();
     l += swap[(half ^ 1) * kM + r_own];
-    if (ok) ok = __all_sync(0xffffffffu, bar_wait(pv_done, (n - 1) & 1));
+    Values::at_end(n, value);
     if (ok) {
       fence_after();
       const float f = __fdiv_rn(1.0f, l) * (spec.head_gate && row < T ? head_sigmoid(p.in[(size_t)row * p.in_ld + spec.gate_row0() + h]) : 1.0f);

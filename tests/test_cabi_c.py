@@ -57,13 +57,13 @@ def test_hot_path_from_plain_c(tmp_path):
     assert "hot path ok" in r.stdout
 
 
-def _compile_xchg_model(tmp_path):
+def _compile_model(tmp_path, name):
     gxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else shutil.which("g++")
     if not gxx:
         pytest.skip("no C++ compiler")
-    exe = str(tmp_path / "xchg_model")
+    exe = str(tmp_path / name)
     subprocess.run([gxx, "-O2", "-std=c++17", "-pthread", "-Wall", "-Werror", "-I", os.path.join(ROOT, "nfai_b200", "csrc"),
-                    os.path.join(ROOT, "tests", "cabi", "xchg_model.cpp"), "-o", exe], check=True)
+                    os.path.join(ROOT, "tests", "cabi", name + ".cpp"), "-o", exe], check=True)
     return exe
 
 
@@ -71,13 +71,25 @@ def _compile_xchg_model(tmp_path):
 def test_exchange_protocol_with_cpu_threads_as_ranks(tmp_path, world, rounds, H):
     """The epoch / parity protocol of the tensor-parallel exchange (the header the kernels compile) run by CPU threads:
     bit-identical sums on every rank, lowest-index arg-max, epochs across the 32-bit wrap."""
-    exe = _compile_xchg_model(tmp_path)
+    exe = _compile_model(tmp_path, "xchg_model")
     r = subprocess.run([exe, str(world), str(rounds), str(H)], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, (r.stdout, r.stderr)
 
 
 def test_exchange_protocol_gives_up_when_a_rank_is_gone(tmp_path):
     """A rank that stops publishing: the others leave their bounded wait with a time-out, nothing hangs."""
-    exe = _compile_xchg_model(tmp_path)
+    exe = _compile_model(tmp_path, "xchg_model")
     r = subprocess.run([exe, "4", "100", "64", "2", "37"], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, (r.stdout, r.stderr)
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+def test_prompt_attention_sees_every_phase_of_its_barriers(tmp_path, kind):
+    """The waits of the softmax warps (the header the kernels compile) in every order in which products, arrivals and warps can
+    proceed: no sum is touched while a product is on its way, no wait is without end, no arrival outlives the CTA."""
+    exe = _compile_model(tmp_path, "attn_phases_model")
+    for tiles in (1, 2, 3, 4, 5, 8, 9):
+        r = subprocess.run([exe, str(kind), str(tiles)], capture_output=True, text=True, timeout=60)
+        assert r.returncode == 0, (tiles, r.stdout, r.stderr)
+    if kind != 2:  # the model sees it where phases that other barriers vouch for are passed over
+        assert subprocess.run([exe, str(kind), "6", "skip"], capture_output=True, timeout=60).returncode == 1
