@@ -184,6 +184,12 @@ struct Step {
   __device__ __forceinline__ void wait(unsigned long long& bar, uint32_t parity, unsigned long long limit = 4 * kGiveUpNs) const {  // (polls may take kGiveUpNs before)
     if (!bar_try(s_addr(&bar), parity)) wait_slowly(sh, sh.p.state, s_addr(&bar), parity, limit);
   }
+  // For roles of a whole warp, whose lanes stay together: one answer. False: a wait on a barrier has given up, nothing is issued any more.
+  __device__ __forceinline__ bool warp_wait(unsigned long long& bar, uint32_t parity) const {
+    if (__all_sync(0xffffffffu, bar_try(s_addr(&bar), parity))) return true;
+    wait_slowly(sh, sh.p.state, s_addr(&bar), parity, 4 * kGiveUpNs);
+    return !__any_sync(0xffffffffu, dead(sh) >= 2);
+  }
   // N pairs of words, kPiece elements apart from `first` on; those from `left` elements on read as zero
   template <int N>
   __device__ __forceinline__ void poll(const uint2* first, uint32_t left, float2 (&v)[N]) const {
@@ -241,11 +247,11 @@ __device__ __forceinline__ void issue_products(const Step& st) {
   Shared& sh = st.sh;
   constexpr uint32_t idesc = (1u << 4) | (kAccColumns >> 3) << 17 | (128u >> 4) << 24;
   const uint64_t a0 = umma::smem_desc_sw128(st.ring), b0 = umma::smem_desc_sw128(st.xs);  // (addresses in units of 16 bytes, below 2^14)
-  const uint32_t tmem = sh.tmem, full = s_addr(&sh.full[0]), empty = s_addr(&sh.empty[0]);
+  const uint32_t tmem = sh.tmem, empty = s_addr(&sh.empty[0]);
   Cursor w, x0, acc;             // weights, the chunk's first piece of x, accumulators
   const uint32_t end = p.L * 4 + (p.with_head ? 1 : 0);
 #pragma unroll 1
-  for (uint32_t k = 0; k < end && dead(sh) < 2; ++k) {
+  for (uint32_t k = 0; k < end; ++k) {
     const Share& s = sh.share[k < p.L * 4 ? k & 3u : (uint32_t)PH_HEAD];
     const uint32_t rows = s.rows, pieces = s.pieces, chunk = chunk_of(s);
 #pragma unroll 1
@@ -256,15 +262,11 @@ __device__ __forceinline__ void issue_products(const Step& st) {
         const uint32_t d = tmem + acc.slot * kAccColumns;
         const bool last = r + kTileRows >= rows;
         Cursor x = x0;
-        st.wait(sh.acc_empty[acc.slot], acc.turn ^ 1u);
+        if (!st.warp_wait(sh.acc_empty[acc.slot], acc.turn ^ 1u)) return;
 #pragma unroll 1
         for (uint32_t i = 0; i < n; ++i, w.next(kSlots), x.next(kXSlots)) {
-          if (r == 0) st.wait(sh.x_full[x.slot], x.turn);
-          if (!bar_try(full + 8 * w.slot, w.turn)) {
-            wait_slowly(sh, p.state, full + 8 * w.slot, w.turn, 4 * kGiveUpNs);
-            if (__any_sync(0xffffffffu, dead(sh) >= 2)) return;
-          }
-          __syncwarp();
+          if (r == 0 && !st.warp_wait(sh.x_full[x.slot], x.turn)) return;
+          if (!st.warp_wait(sh.full[w.slot], w.turn)) return;
           umma::fence_after();
           if (umma::elect_one()) {
             const uint64_t a = a0 + w.slot * (kSlotBytes / 16), b = b0 + x.slot * (kXBytes / 16);
