@@ -99,10 +99,11 @@ int nfai_tp_import_peers(nfai_ctx* ctx, const void* descs, int n);
 /* replaces: LlamaModelFactory.Dispose (LlamaModelFactory.cs:24-32). */
 int nfai_ctx_destroy(nfai_ctx* ctx);
 
-/* Budget, in nanoseconds, of every device-side wait on another rank (exchange flags). Default one second, or the
- * environment variable NFAI_WAIT_NS at context creation. A wait that runs out makes the call return
- * NFAI_ERR_TIMEOUT; the kernel itself always returns. Takes effect for graphs captured afterwards
- * (nfai_model_finalize, nfai_model_tune).
+/* Budget, in nanoseconds, of every device-side wait on another rank (exchange words) and, where a decode step is one
+ * resident kernel (nfai_step_kernels), of its CTAs' waits on one another. Default one second, or the environment
+ * variable NFAI_WAIT_NS at context creation. A wait that runs out makes the call return NFAI_ERR_TIMEOUT; the kernel
+ * itself always returns, and the cache row of that step is not valid (nfai_set_position goes back). Takes effect for
+ * graphs captured afterwards (nfai_model_finalize, nfai_model_tune) and for the next resident step.
  * replaces: nothing -- the reference waits on a fence without limit (VulkanBufferManager.cs:474-494). */
 int nfai_ctx_set_wait_ns(nfai_ctx* ctx, uint64_t ns);
 

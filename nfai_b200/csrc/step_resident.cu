@@ -16,8 +16,9 @@
 // Hand-overs go through memory words of (value, tag), as between the ranks of a tensor-parallel group (xchg_protocol.h): a row's
 // result is one 8-byte store, a reader polls the words it needs until each carries this step's tag. No flag, no fence, no
 // barrier across the grid. Every phase of every layer has words of its own, so a word is written once per step, and the tag is the
-// number of the step. All CTAs are on the GPU at the same time, so a poll ends; should it not, it gives up after a second
-// (error bit 4 of the step state, NFAI_ERR_TIMEOUT) and the kernel runs to its end without waiting again.
+// number of the step. All CTAs are on the GPU at the same time, so a poll ends; should it not within the context's budget
+// (nfai_ctx_set_wait_ns), it gives up (error bit 4 of the step state, NFAI_ERR_TIMEOUT) and the kernel runs to its end without waiting
+// for results again. It does wait, with a limit of its own, for what is on its way into a CTA's memory before that CTA leaves.
 //
 // Split of the work. Rows of every matrix are dealt evenly over the CTAs in contiguous blocks. A ring slot holds a tile of 16 rows
 // and 512 columns, eight blocks of 64; warp b makes the terms of block b of every piece of x: it polls exactly those columns, and no
@@ -57,7 +58,8 @@ constexpr uint32_t kAcc = 8, kAccColumns = 32;    // accumulators in tensor memo
 constexpr uint32_t kBlockRows = 128;              // rows whose sums meet in shared memory at a time
 constexpr uint32_t kPartFloats = 2 * kBlockRows * 4;  // two buffers of four warps' sums
 constexpr uint32_t kMaxNarrow = kNarrow * kPiece, kMaxWide = 16384;
-constexpr unsigned long long kGiveUpNs = 1000000000ull;
+constexpr unsigned long long kLeaveNs = 1000000000ull;     // a CTA that leaves: for its copies and products to end
+constexpr unsigned long long kArrivalsNs = 100000ull;      // ... and, where waits have given up, for arrivals that nobody counts
 
 // ---- barriers, copies, words ---------------------------------------------------------------------------------------------
 using umma::bar_arrive;
@@ -137,7 +139,6 @@ __device__ __forceinline__ void give_up(Shared& sh, StepState* state, uint32_t h
   atomicMax(&sh.dead, how);
   atomicOr(&state->err, 4u);
 }
-// Not inlined: what a layer executes has to stay in the instruction cache (below).
 __device__ __forceinline__ void wait_slowly(Shared& sh, StepState* state, uint32_t bar, uint32_t parity, unsigned long long limit) {
   const unsigned long long t0 = global_timer_ns();
   for (uint32_t polls = 1; !bar_try(bar, parity) && dead(sh) < 2; ++polls)
@@ -156,10 +157,10 @@ __device__ __forceinline__ void poll_words(Shared& sh, StepState* state, uint32_
 #pragma unroll
     for (int j = 0; j < N; ++j) all = all && w[j].y == tag && w[j].w == tag;
     if (all) return;
-    if ((polls & 63u) == 1) {
+    if ((polls & 3u) == 1) {
       if (dead(sh)) return;
       if (t0 == 0) t0 = global_timer_ns();
-      else if (global_timer_ns() - t0 > kGiveUpNs) return give_up(sh, state, 1);
+      else if (global_timer_ns() - t0 > sh.p.wait_ns) return give_up(sh, state, 1);
     }
   }
 }
@@ -181,13 +182,19 @@ struct Step {
   float* const work;             // the warps' attention states
   float* const part;             // row sums
 
-  __device__ __forceinline__ void wait(unsigned long long& bar, uint32_t parity, unsigned long long limit = 4 * kGiveUpNs) const {  // (polls may take kGiveUpNs before)
-    if (!bar_try(s_addr(&bar), parity)) wait_slowly(sh, sh.p.state, s_addr(&bar), parity, limit);
+  // (four times the budget: what arrives here may have polled for words before)
+  __device__ __forceinline__ void wait(unsigned long long& bar, uint32_t parity) const {
+    if (!bar_try(s_addr(&bar), parity)) wait_slowly(sh, sh.p.state, s_addr(&bar), parity, 4 * sh.p.wait_ns);
+  }
+  // For a CTA that leaves: whether or not waits have given up.
+  __device__ __forceinline__ void wait_out(unsigned long long& bar, uint32_t parity) const {
+    const unsigned long long t0 = global_timer_ns();
+    while (!bar_try(s_addr(&bar), parity) && global_timer_ns() - t0 < kLeaveNs) {}
   }
   // For roles of a whole warp, whose lanes stay together: one answer. False: a wait on a barrier has given up, nothing is issued any more.
   __device__ __forceinline__ bool warp_wait(unsigned long long& bar, uint32_t parity) const {
     if (__all_sync(0xffffffffu, bar_try(s_addr(&bar), parity))) return true;
-    wait_slowly(sh, sh.p.state, s_addr(&bar), parity, 4 * kGiveUpNs);
+    wait_slowly(sh, sh.p.state, s_addr(&bar), parity, 4 * sh.p.wait_ns);
     return !__any_sync(0xffffffffu, dead(sh) >= 2);
   }
   // N pairs of words, kPiece elements apart from `first` on; those from `left` elements on read as zero
@@ -703,11 +710,11 @@ __device__ __forceinline__ void feed(const Step& st, const ResidentStep& launch)
         for (uint32_t piece = c0; piece < min(s.pieces, c0 + chunk); ++piece, ++begun, c.next(kSlots)) {
           const uint32_t full = s_addr(&sh.full[c.slot]);
           if (begun >= kAhead) {
-            st.wait(sh.full[landed.slot], landed.turn, kGiveUpNs);
+            if (!st.warp_wait(sh.full[landed.slot], landed.turn)) goto drain;
             landed.next(kSlots);
             ++seen;
           }
-          if (begun >= kSlots) st.wait(sh.empty[c.slot], c.turn ^ 1u);
+          if (begun >= kSlots && !st.warp_wait(sh.empty[c.slot], c.turn ^ 1u)) goto drain;
           if (__any_sync(0xffffffffu, dead(sh) >= 2)) goto drain;  // nothing more goes into a slot that may still be read or written
           if (umma::elect_one()) {
             bar_expect_tx(full, rows * (kPiece * 2));
@@ -728,9 +735,9 @@ __device__ __forceinline__ void feed(const Step& st, const ResidentStep& launch)
     }
   }
 drain:  // nothing is on its way into this CTA's memory when it leaves, neither copies nor the products' arrivals on the slots' barriers
-  for (; seen < begun; ++seen, landed.next(kSlots)) st.wait(sh.full[landed.slot], landed.turn, kGiveUpNs);
-  if (dead(sh) < 2) {
-    for (uint32_t i = 0; i < min(begun, kSlots); ++i) st.wait(sh.empty[i], (begun - 1 - i) / kSlots & 1u, kGiveUpNs);
+  for (; seen < begun; ++seen, landed.next(kSlots)) st.wait_out(sh.full[landed.slot], landed.turn);
+  if (dead(sh) < 2) {  // (else the products of the last copies may never have been issued: kArrivalsNs)
+    for (uint32_t i = 0; i < min(begun, kSlots); ++i) st.wait_out(sh.empty[i], (begun - 1 - i) / kSlots & 1u);
   }
 }
 
@@ -796,8 +803,11 @@ __global__ void __launch_bounds__(kAllThreads, 1) step_resident_kernel(const __g
     // the last products, and their arrivals on the barriers of x, before the memory goes
     if (umma::elect_one()) umma::umma_commit(s_addr(&sh.drained));
     __syncwarp();
-    const unsigned long long t0 = global_timer_ns();
-    while (!bar_try(s_addr(&sh.drained), 0) && global_timer_ns() - t0 < kGiveUpNs) {}
+    st.wait_out(sh.drained, 0);
+    if (dead(sh) >= 2) {  // arrivals of products that are done, on barriers that are not waited for any more
+      const unsigned long long t0 = global_timer_ns();
+      while (global_timer_ns() - t0 < kArrivalsNs) {}
+    }
   } else {
     {  // this CTA's columns of the embedding row
       const uint32_t i = 2 * tid, at = sh.share[PH_O].row0 + i;
@@ -820,7 +830,7 @@ __global__ void __launch_bounds__(kAllThreads, 1) step_resident_kernel(const __g
       sync();
     }
     if (warp == 0 && dead(sh) < 2)  // (the products' arrivals on the last pieces of x)
-      for (uint32_t i = 0; i < kXSlots; ++i, xc.next(kXSlots)) st.wait(sh.x_empty[xc.slot], xc.turn ^ 1u, kGiveUpNs);
+      for (uint32_t i = 0; i < kXSlots; ++i, xc.next(kXSlots)) st.wait_out(sh.x_empty[xc.slot], xc.turn ^ 1u);
   }
 
   umma::fence_before();

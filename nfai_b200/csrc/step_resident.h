@@ -26,6 +26,7 @@ struct ResidentArgs {
   uint32_t* epoch = nullptr;            // steps so far
   uint32_t* ticket = nullptr;           // zero between steps
   uint32_t with_head = 1;
+  unsigned long long wait_ns = 1000000000ull;  // budget of a poll
   // filled in by resident_plan
   uint32_t words_per_layer = 0, splits = 1;
 };

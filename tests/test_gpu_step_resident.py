@@ -2,7 +2,7 @@
 import numpy as np
 import pytest
 
-from nfai_b200 import LlamaModelFactory, create_synthetic_model, synth
+from nfai_b200 import LlamaModelFactory, NfaiError, _lib, create_synthetic_model, synth
 
 from .test_gpu_prompt_exact import PlainLlama, off
 
@@ -112,3 +112,35 @@ def test_extreme_inputs(factory):
         m.Dispose()
     assert np.isfinite(logits[0][0]).all() and float(np.linalg.norm(logits[0][0] - logits[1][0]) / np.linalg.norm(logits[1][0])) < 1e-5
     assert not np.isfinite(logits[0][1]).any() and not np.isfinite(logits[1][1]).any()
+
+
+def test_a_wait_that_runs_out_is_a_status(factory):
+    """With a budget of a nanosecond a step's CTAs give up on one another: the kernel returns, the call says so, and nothing of it is
+    left for the next step. Launches have nothing to wait for."""
+    def budget(ns):
+        _lib.check(_lib.load().nfai_ctx_set_wait_ns(factory.ctx.handle, ns), factory.ctx.handle)
+
+    cfg = synth.get_config("s1", V=2053)
+    m, launches = (create_synthetic_model(c, 256, factory=factory) for c in (cfg, synth.get_config("c0")))
+    assert m.step_kernels() == 1 and launches.step_kernels() > 1
+    ids = synth.prompt_ids(cfg, 20, 3)
+    m.prefill(ids)
+    want = m.decode(7)[0]
+    answer, _ = m.decode_greedy(9, 6)
+    small = launches.decode(7)[0]
+    try:
+        budget(1)
+        for _ in range(4):
+            m.set_position(len(ids))
+            with pytest.raises(NfaiError) as e:
+                m.decode(7)
+            assert e.value.code == _lib.ERR_TIMEOUT
+        launches.reset()
+        assert np.array_equal(launches.decode(7)[0], small)
+    finally:
+        budget(1_000_000_000)
+    m.set_position(len(ids))
+    assert np.array_equal(m.decode(7)[0], want)
+    assert list(m.decode_greedy(9, 6)[0]) == list(answer)
+    m.Dispose()
+    launches.Dispose()

@@ -140,8 +140,8 @@ def test_a_pull_without_its_peer_times_out_and_the_context_survives(cuda_ctx, or
 
 
 def test_a_model_step_reports_a_timeout_as_a_status(cuda_ctx):
-    """nfai_ctx_set_wait_ns is accepted, rejects zero, and a one-GPU model keeps working with a tiny budget (it has no
-    waits on peers to run out)."""
+    """nfai_ctx_set_wait_ns is accepted and rejects zero. (What a tiny budget does to the steps of one-GPU models:
+    test_gpu_step_resident.py.)"""
     lib = _lib.load()
     assert lib.nfai_ctx_set_wait_ns(cuda_ctx.handle, 0) == _lib.ERR_ARG
     assert lib.nfai_ctx_set_wait_ns(cuda_ctx.handle, 1000) == _lib.OK
