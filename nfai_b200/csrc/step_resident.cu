@@ -269,10 +269,11 @@ __device__ __forceinline__ void issue_products(const Step& st) {
         const uint32_t d = tmem + acc.slot * kAccColumns;
         const bool last = r + kTileRows >= rows;
         Cursor x = x0;
-        if (!st.warp_wait(sh.acc_empty[acc.slot], acc.turn ^ 1u)) return;
+        st.wait(sh.acc_empty[acc.slot], acc.turn ^ 1u);
 #pragma unroll 1
         for (uint32_t i = 0; i < n; ++i, w.next(kSlots), x.next(kXSlots)) {
-          if (r == 0 && !st.warp_wait(sh.x_full[x.slot], x.turn)) return;
+          // (one decision a piece: with votes behind the other two waits as well the 1B architecture took 486.6 us a step, 481.5 so)
+          if (r == 0) st.wait(sh.x_full[x.slot], x.turn);
           if (!st.warp_wait(sh.full[w.slot], w.turn)) return;
           umma::fence_after();
           if (umma::elect_one()) {
