@@ -370,12 +370,12 @@ int capture(nfai_model* m, bool with_head, bool from_prompt, cudaGraphExec_t* ou
   return NFAI_OK;
 }
 
-// Whether the step runs as one resident kernel, and its layout. One GPU, caches of up to 4 096 positions (beyond, attention is most
-// of the step and runs on the tensor cores), and no launch shape asked for.
+// Whether the step can run as one resident kernel, and its layout. One GPU, caches of up to 4 096 positions (beyond, attention is most
+// of the step and runs on the tensor cores).
 bool plan_resident(nfai_model* m) {
   nfai_ctx* c = m->ctx;
   const nfai_hparams& hp = m->hp;
-  if (c->world != 1 || !c->use_graph || m->shaped || hp.ctx > 4096 || m->attn_heads != 1) return false;
+  if (c->world != 1 || !c->use_graph || hp.ctx > 4096 || m->attn_heads != 1) return false;
   ResidentStep& p = m->step;
   p.L = hp.L; p.H = hp.H; p.qH = hp.qH; p.kvH = hp.kvH; p.d = hp.d; p.F = hp.F; p.V = hp.V; p.ctx = hp.ctx; p.ropeDim = hp.ropeDim;
   p.eps = hp.eps;
@@ -413,10 +413,15 @@ void bind_resident(nfai_model* m, char* words, char* counts) {
   p.ticket = p.epoch + 1;
 }
 
+// Whether the step at position `pos` is one kernel: launch shapes and an L2 look-ahead belong to a sequence of launches.
+bool steps_resident(const nfai_model* m, uint32_t pos) {
+  return m->resident && !m->shaped && !m->pf_look && !m->pf_extra && pos < resident_positions(m->hp.d);
+}
+
 // The step at position `pos`: where the model stands when it runs.
 int run_step(nfai_model* m, bool with_head, bool from_prompt, uint32_t pos) {
   nfai_ctx* c = m->ctx;
-  if (m->resident && pos < resident_positions(m->hp.d)) {
+  if (steps_resident(m, pos)) {
     ResidentStep p = m->step;
     p.with_head = with_head ? 1 : 0;
     p.prompt = from_prompt ? m->prompt : nullptr;
@@ -1524,8 +1529,10 @@ int nfai_model_tune(nfai_model* m, int which, int mode, int rows_per_warp, int d
   t->ctas_per_sm = ctas_per_sm;
   t->grid = grid;
   t->split = split;
-  m->shaped = true;
-  if (!m->finalized) return NFAI_OK;
+  if (!m->finalized) {
+    m->shaped = true;
+    return NFAI_OK;
+  }
   CU(c, cudaSetDevice(c->device));
   CU(c, cudaStreamSynchronize(c->stream));
   if (which == 4) {
@@ -1539,7 +1546,7 @@ int nfai_model_tune(nfai_model* m, int which, int mode, int rows_per_warp, int d
   }
   int rc = capture_graphs(m);
   if (rc != NFAI_OK) *t = old;
-  else m->resident = false;
+  else m->shaped = true;
   return rc;
 }
 
@@ -1551,13 +1558,10 @@ int nfai_model_set_prefetch(nfai_model* m, uint64_t lookahead_bytes, uint64_t ex
   m->pf_look = lookahead_bytes;
   m->pf_extra = extra_bytes;
   m->pf_mode = mode;
-  m->shaped = true;
   if (!m->finalized || !c->use_graph) return NFAI_OK;
   CU(c, cudaSetDevice(c->device));
   CU(c, cudaStreamSynchronize(c->stream));
-  int rc = capture_graphs(m);
-  if (rc == NFAI_OK) m->resident = false;
-  return rc;
+  return capture_graphs(m);
 }
 
 int nfai_step_launches(const nfai_model* m, int* out) {
@@ -1568,7 +1572,7 @@ int nfai_step_launches(const nfai_model* m, int* out) {
 
 int nfai_step_kernels(const nfai_model* m, int* out) {
   int rc = nfai_step_launches(m, out);
-  if (rc == NFAI_OK && m->resident && m->pos < resident_positions(m->hp.d)) *out = 1;
+  if (rc == NFAI_OK && steps_resident(m, m->pos)) *out = 1;
   return rc;
 }
 

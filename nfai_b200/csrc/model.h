@@ -132,8 +132,8 @@ struct nfai_model {
   void* sample_scratch = nullptr;  // per-slice sums and candidates of the on-device sampler
   cudaGraphExec_t g_full = nullptr, g_nohead = nullptr;
   int launches_full = 0;
-  bool shaped = false;    // launch shapes or the L2 look-ahead were asked for: the step is the sequence of launches they belong to
-  bool resident = false;  // the step is one kernel (step_resident.cu)
+  bool shaped = false;    // launch shapes were asked for: the step is the sequence of launches they belong to
+  bool resident = false;  // the step can be one kernel (step_resident.cu); whether it is: steps_resident in api.cu
   ResidentStep step;
   uint32_t pos = 0;  // host mirror of state->pos
   GemvTune tune_qkv, tune_o, tune_gateup, tune_down, tune_head;

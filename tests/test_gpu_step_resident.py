@@ -144,3 +144,24 @@ def test_a_wait_that_runs_out_is_a_status(factory):
     assert list(m.decode_greedy(9, 6)[0]) == list(answer)
     m.Dispose()
     launches.Dispose()
+
+
+def test_a_look_ahead_runs_the_launches_it_belongs_to(factory, monkeypatch):
+    """Asked for by a call or from outside, and only as long as it is."""
+    cfg = synth.get_config("s1", V=2053)
+    m = create_synthetic_model(cfg, 64, factory=factory)
+    first = m.decode(3)[0]
+    for look, extra in ((1 << 20, 0), (0, 1 << 20), (0, 0)):
+        m.set_prefetch(look, extra)
+        assert (m.step_kernels() == 1) == (look + extra == 0) and m.step_launches() > 1
+    m.reset()
+    assert np.array_equal(m.decode(3)[0], first)
+    m.Dispose()
+    for name in ("NFAI_PF_MB", "NFAI_PF_EXTRA_MB"):
+        monkeypatch.setenv(name, "1")
+        m = create_synthetic_model(cfg, 64, factory=factory)
+        monkeypatch.delenv(name)
+        assert m.step_kernels() == m.step_launches()
+        m.set_prefetch(0)
+        assert m.step_kernels() == 1
+        m.Dispose()
