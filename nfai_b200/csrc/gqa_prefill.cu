@@ -495,7 +495,7 @@ cudaError_t launch_gqa_prep(cudaStream_t s, const GqaParams& p, uint32_t T) {
 cudaError_t launch_gqa_prefill(cudaStream_t s, const GqaParams& p, uint32_t T) {
   if (!T || !p.in || !p.q || !p.ao || (uint64_t)p.pos0 + T > p.ctx) return cudaErrorInvalidValue;
   const int kind = env_int("NFAI_PREFILL_ATTN", 1);
-  if (kind == 1 && gqa_prefill_umma_supported(p, T)) return launch_gqa_prefill_umma(s, p, T);
+  if (kind != 0 && kind != 2 && gqa_prefill_umma_supported(p, T)) return launch_gqa_prefill_umma(s, p, T);
   if (p.dtype == 2 && kind != 0 && mma_supported(p.spec)) {
     const uint32_t dim = p.spec.dim, dv = value_width(p.spec.vdim);
     if (dim > 32 && dim <= 64 && dv == 64) return launch_mma<64, 64, 64>(s, p, T);

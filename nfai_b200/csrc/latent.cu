@@ -530,8 +530,7 @@ cudaError_t launch_latent_prefill_mma(cudaStream_t s, const LatentParams& p, uin
 
 cudaError_t launch_latent_prefill(cudaStream_t s, const LatentParams& p, uint32_t T) {
   if (!T || p.spec.heads > 65535) return cudaErrorInvalidValue;
-  static const bool mma_on = env_int("NFAI_PREFILL_ATTN", 1) != 0;
-  if (p.dtype == 2 && mma_on && latent_prefill_mma_supported(p.spec)) return launch_latent_prefill_mma(s, p, T);
+  if (p.dtype == 2 && env_int("NFAI_PREFILL_ATTN", 1) != 0 && latent_prefill_mma_supported(p.spec)) return launch_latent_prefill_mma(s, p, T);
   const size_t smem = (size_t)(p.spec.dim + p.spec.rot + p.spec.vdim + kSB) * 4;
   const dim3 grid(T, p.spec.heads);
   if (p.dtype == 0) return launch_pdl(latent_prefill_simt_kernel<float>, grid, dim3(kST), smem, s, prefill_pdl(), p);

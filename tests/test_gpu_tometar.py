@@ -481,3 +481,19 @@ def test_bfloat16_gemv(cuda_ctx, N, K):
     x64 = x.astype(np.float64)
     ref = W.astype(np.float64) @ (x64 / np.sqrt((x64 * x64).mean() + 1e-5) * gain) + res
     assert np.abs(host(y) - ref).max() < 2e-4
+
+
+def test_every_prompt_pass_reads_its_switch(cuda_ctx, monkeypatch):
+    """One model, the tensor-core and the any-size kernel in turn: other bits, both right."""
+    cfg = U.config([U.layer(U.latent(4, 32, 16, 48, 64, 40), 144)], 112, 200, 1)
+    W = U.weights(cfg, 9)
+    toks = list(range(100))
+    want = P.forward(cfg, {k: v.astype(np.float64) for k, v in W.items()}, toks)
+    m, got = build(cuda_ctx, cfg, W, "bf16"), []
+    for kind in ("1", "0", "1"):
+        monkeypatch.setenv("NFAI_PREFILL_ATTN", kind)
+        m.reset()
+        got.append(m.forward(toks, range(len(toks))))
+        assert U.error(got[-1], want) < TOL["bf16"]
+    m.Dispose()
+    assert np.array_equal(got[0], got[2]) and not np.array_equal(got[0], got[1])
