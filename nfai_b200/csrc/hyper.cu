@@ -156,9 +156,12 @@ cudaError_t launch_st(cudaStream_t s, const HyperRows& p, uint32_t n) {
     if (p.H % 4 == 0) kern = hyper_rows_kernel<ST, 4, 256>;
   }
   if constexpr (ST <= 4) {
-    // Rows wider than 256 quads: all of a row of 2048 is in flight at once, on 1024 threads of an SM (256 a CTA and 768: 35.0 us for
-    // the 159 MB of 2011 tokens of 4 streams, 512: 29.9, 5.3 TB/s).
-    if (p.H % 4 == 0 && p.H > 1024) {
+    // Rows wider than 256 quads that all find room at once, two CTAs an SM: what counts is how long one row takes. More rows keep an SM's
+    // 1024 threads busy either way, and smaller CTAs end less together. Measured, us (256 threads, 512; before both 256 threads, 768 on an
+    // SM), 4 streams of 2048: 37 rows 12.3, 10.2 (12.3), 296: 14.4, 14.3 (16.4), 360: 14.4, 16.4 (16.4), 2011: 41.0, 43.0 (51.2), 8192: 123,
+    // 139 (162); of 8192: 296 rows 30.7, 28.7 (34.9), 592: 45.1, 47.1 (67.6), 2011: 139, 133 (168); 1 stream of 1028: 37 rows 10.2, 8.3
+    // (10.3), 2011: 19.5, 24.6 (20.5).
+    if (p.H % 4 == 0 && p.H > 1024 && n <= 2 * sm_count()) {
       kern = hyper_rows_kernel<ST, 4, 512>;
       threads = 512;
     }

@@ -215,6 +215,27 @@ def test_a_rows_norm_does_not_depend_on_the_threads(cuda_ctx, streams, width):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("width,streams", [(1028, 1), (2048, 4)])
+def test_rows_do_not_depend_on_how_many_there_are(cuda_ctx, width, streams):
+    """Few rows are read by wider CTAs than many (the line is at two rows an SM): the same bits on both sides of it. In 32 bits the
+    products and the recurrence have one order for any number of rows."""
+    cfg = U.config([U.layer(U.ssm(2, 16, 8, 1, 3, 2), 40), U.layer(U.ssm(2, 16, 8, 1, 3, 2))], width, 64, streams)
+    W = U.weights(cfg, 5)
+    m = build(cuda_ctx, cfg, W, "f32", 640)
+    line = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    toks, places = np.random.default_rng(width).integers(0, 64, 2 * line).tolist(), range(0, 2 * line, 9)
+    got = []
+    for portions in ((line, line), (line + 1, line - 1), (2 * line,)):
+        m.reset()
+        at, rows = 0, []
+        for n in portions:
+            rows += list(m.forward(toks[at:at + n], [p - at for p in places if at <= p < at + n]))
+            at += n
+        got.append(np.array(rows))
+    m.Dispose()
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+
+
 @pytest.mark.parametrize("streams", [1, 2, 5, 8, 9, 16])
 def test_stream_counts(cuda_ctx, streams):
     cfg = U.config([U.layer(U.latent(2, 16, 8, 16, 24, 9), 40), U.layer(U.ssm(2, 16, 8, 1, 3, 2))], 48, 40, streams)
