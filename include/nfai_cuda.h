@@ -290,7 +290,7 @@ int nfai_model_set_prefetch(nfai_model* m, uint64_t lookahead_bytes, uint64_t ex
 int nfai_step_launches(const nfai_model* m, int* out);
 
 /* Number of kernels that the step at the current position launches: 1 where the whole step is one resident kernel (float16
- * models of some size on one GPU, caches of up to 4 096 positions, no launch shapes or look-ahead asked for), else as above. */
+ * models of some size with a float16 cache of up to 4 096 positions on one GPU, no launch shapes or look-ahead asked for), else as above. */
 int nfai_step_kernels(const nfai_model* m, int* out);
 
 /* ---- single kernels on caller-owned DEVICE buffers (kernel-level parity tests, embedding in other hosts) - */

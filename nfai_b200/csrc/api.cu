@@ -426,7 +426,7 @@ int run_step(nfai_model* m, bool with_head, bool from_prompt, uint32_t pos) {
     p.with_head = with_head ? 1 : 0;
     p.prompt = from_prompt ? m->prompt : nullptr;
     p.wait_ns = std::min(c->wait_ns, 1ull << 60);
-    CU(c, launch_step_resident(c->stream, m->hp.kv_dtype, p));
+    CU(c, launch_step_resident(c->stream, p));
     return NFAI_OK;
   }
   if (c->use_graph) {

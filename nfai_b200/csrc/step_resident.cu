@@ -1,5 +1,6 @@
 // A decode step as ONE kernel that stays on the GPU from the embedding row to the arg-max: one CTA per SM, all resident
-// (cooperative launch), the layers' products and attentions as phases of a loop. Models with float16 weights on one GPU.
+// (cooperative launch), the layers' products and attentions as phases of a loop. Models with float16 weights and a float16 cache on one
+// GPU.
 //
 // What bounds a step is the stream of its weights out of HBM; what a step made of launches loses on top are its hand-overs: five a
 // layer at about 2 us each (the wait for the last CTA, then x out of L2), during which only what a kernel requested before its
@@ -11,7 +12,8 @@
 // the warps it was not: 25 bytes, half of the instructions conversions and sums across lanes, 549 us a step of the 1B architecture;
 // with warp-level products 39 bytes and 548 us. So tcgen05 multiplies, exactly: float16 weights are the A operand as they lie in the
 // ring, x is split into three float16 terms of 11 bits each, scaled to the largest element of its block, as the B operand. Every
-// product is exact and sums are float32 in tensor memory; one thread issues them, and no warp touches a weight.
+// product is exact and sums are float32 in tensor memory (resident_plan says what they lose); one thread issues them, and no warp
+// touches a weight.
 //
 // Hand-overs go through memory words of (value, tag), as between the ranks of a tensor-parallel group (xchg_protocol.h): a row's
 // result is one 8-byte store, a reader polls the words it needs until each carries this step's tag. No flag, no fence, no
@@ -299,9 +301,9 @@ __device__ __forceinline__ uint32_t words_mid(const ResidentArgs& p) { return wo
 __device__ __forceinline__ uint32_t words_hid(const ResidentArgs& p) { return words_mid(p) + p.H; }
 __device__ __forceinline__ uint32_t words_out(const ResidentArgs& p) { return words_hid(p) + p.F; }
 __device__ __forceinline__ uint32_t words_part(const ResidentArgs& p) { return words_out(p) + p.H; }
-template <typename KVT, int D>
-__device__ __forceinline__ KVT* layer_cache(const ResidentArgs& p, void* cache, uint32_t l) {
-  return reinterpret_cast<KVT*>(cache) + (size_t)l * p.ctx * (p.kvH * D);
+template <int D>
+__device__ __forceinline__ __half* layer_cache(const ResidentArgs& p, void* cache, uint32_t l) {
+  return reinterpret_cast<__half*>(cache) + (size_t)l * p.ctx * (p.kvH * D);
 }
 
 // The lowest index among the maxima.
@@ -314,7 +316,7 @@ __device__ __forceinline__ void take_best(float& v, uint32_t& i, float ov, uint3
 
 // The pair of rows `row`, `row` + 1 (`local` within the share) of phase `ph` of layer l; both: the second one is a row of this CTA
 // too.
-template <typename KVT, int D>
+template <int D>
 __device__ __forceinline__ void finish_pair(const Step& st, uint32_t l, uint32_t ph, uint32_t row, uint32_t local, float a, float b, bool both) {
   const ResidentArgs& p = st.sh.p;
   Shared& sh = st.sh;
@@ -330,7 +332,7 @@ __device__ __forceinline__ void finish_pair(const Step& st, uint32_t l, uint32_t
     }
     if (row >= qDim && sh.keep) {
       const bool key = row < qDim + kvDim;
-      KVT* k = layer_cache<KVT, D>(p, key ? p.kc : p.vc, l) + (size_t)sh.pos * kvDim + (row - qDim - (key ? 0 : kvDim));
+      __half* k = layer_cache<D>(p, key ? p.kc : p.vc, l) + (size_t)sh.pos * kvDim + (row - qDim - (key ? 0 : kvDim));
       store_as(k, a);
       store_as(k + 1, b);
     }
@@ -462,7 +464,7 @@ __device__ __forceinline__ void take_tile(const Step& st, const Cursor& acc, uin
 }
 
 // The product of this CTA's share in phase ph of layer l with x, and its epilogue.
-template <typename KVT, int D>
+template <int D>
 __device__ __forceinline__ void product(const Step& st, Cursor& xc, Cursor& acc, uint32_t l, uint32_t ph) {
   const ResidentArgs& p = st.sh.p;
   const Share& s = st.sh.share[ph];
@@ -505,33 +507,30 @@ __device__ __forceinline__ void product(const Step& st, Cursor& xc, Cursor& acc,
         v.y += o.y;
       }
       if (t < (n + 1) / 2)
-        finish_pair<KVT, D>(st, l, ph, s.row0 + r0 + 2 * t, ph == PH_HEAD ? t : r0 / 2 + t, __fdiv_rn(v.x, rms), __fdiv_rn(v.y, rms), 2 * t + 1 < n);
+        finish_pair<D>(st, l, ph, s.row0 + r0 + 2 * t, ph == PH_HEAD ? t : r0 / 2 + t, __fdiv_rn(v.x, rms), __fdiv_rn(v.y, rms), 2 * t + 1 < n);
     }
   }
 }
 
 // ---- attention -------------------------------------------------------------------------------------------------------------
 using attn_detail::kNegBig;
-using attn_detail::KV8;
+using KV8 = attn_detail::KV8<__half>;
 // as the cache will hold it
-template <typename KVT>
-__device__ __forceinline__ float as_cached(float v) {
-  if constexpr (sizeof(KVT) == 2) return __half2float(__float2half_rn(v));
-  return v;
-}
+__device__ __forceinline__ float as_cached(float v) { return __half2float(__float2half_rn(v)); }
 
 // Positions a CTA takes before the range is split: two batches of what its lanes request at once. Splitting costs a hand-over
 // (the merge), a batch more about as much.
-constexpr uint32_t attn_batch(uint32_t d, uint32_t kv_bytes) { return kWarps * (32 / (d / 8)) * (kv_bytes == 2 ? 4 : 2); }
+constexpr uint32_t kRequests = 4;  // of a lane, each for keys and values
+constexpr uint32_t attn_batch(uint32_t d) { return kWarps * (32 / (d / 8)) * kRequests; }
 
-template <typename KVT, int D>
+template <int D>
 __device__ __forceinline__ void attention(const Step& st, uint32_t l) {
-  constexpr uint32_t LPP = D / 8, PPW = 32 / LPP, UNR = sizeof(KVT) == 2 ? 4 : 2, NW = kWarps, SSTR = D + 4;  // lanes of a position, positions of a warp
+  constexpr uint32_t LPP = D / 8, PPW = 32 / LPP, UNR = kRequests, NW = kWarps, SSTR = D + 4;  // lanes of a position, positions of a warp
   const ResidentArgs& p = st.sh.p;
   const uint32_t seq = st.sh.pos + 1;
   uint32_t chunk = (seq + p.splits - 1) / p.splits;
-  chunk = max(chunk, attn_batch(D, sizeof(KVT)));
-  if (seq <= 2 * attn_batch(D, sizeof(KVT))) chunk = seq;
+  chunk = max(chunk, attn_batch(D));
+  if (seq <= 2 * attn_batch(D)) chunk = seq;
   const uint32_t S = (seq + chunk - 1) / chunk, items = p.qH * S, kvDim = p.kvH * D;
   float* const wpart = st.work;              // [NW][SSTR]
   float* const qs = st.work + NW * SSTR;     // query, newest key, newest value
@@ -541,16 +540,16 @@ __device__ __forceinline__ void attention(const Step& st, uint32_t l) {
     const uint32_t t1 = min(seq, (s + 1) * chunk), newest = seq - 1;
     const uint32_t tid = thread_id(), lane = tid & 31, warp = tid >> 5, grp = lane / LPP, sub = lane % LPP;
     uint32_t base = s * chunk + warp * PPW;
-    const KVT* kc = layer_cache<KVT, D>(p, p.kc, l) + g * D + sub * 8;
-    const KVT* vc = layer_cache<KVT, D>(p, p.vc, l) + g * D + sub * 8;
-    typename KV8<KVT>::Raw kr[UNR], vr[UNR];
+    const __half* kc = layer_cache<D>(p, p.kc, l) + g * D + sub * 8;
+    const __half* vc = layer_cache<D>(p, p.vc, l) + g * D + sub * 8;
+    KV8::Raw kr[UNR], vr[UNR];
     auto request = [&]() {
 #pragma unroll
       for (uint32_t u = 0; u < UNR; ++u) {
         const uint32_t t = base + u * (NW * PPW) + grp;
         const bool there = t < t1 && t != newest;
-        kr[u] = there ? KV8<KVT>::template ld<true>(kc + (size_t)t * kvDim) : KV8<KVT>::zero();
-        vr[u] = there ? KV8<KVT>::template ld<true>(vc + (size_t)t * kvDim) : KV8<KVT>::zero();
+        kr[u] = there ? KV8::ld<true>(kc + (size_t)t * kvDim) : KV8::zero();
+        vr[u] = there ? KV8::ld<true>(vc + (size_t)t * kvDim) : KV8::zero();
       }
     };
     const float scale = 1.0f / sqrtf((float)D);
@@ -582,7 +581,7 @@ __device__ __forceinline__ void attention(const Step& st, uint32_t l) {
           const uint32_t i = 2 * tid, part = i / D, e = i % D;
           float2 v[1];
           st.poll<1>(layer_words(p, l + 1) + (part == 0 ? h * D : p.qH * D + (part - 1) * kvDim + g * D) + e, 1, v);
-          *reinterpret_cast<float2*>(qs + i) = part == 0 ? v[0] : make_float2(as_cached<KVT>(v[0].x), as_cached<KVT>(v[0].y));
+          *reinterpret_cast<float2*>(qs + i) = part == 0 ? v[0] : make_float2(as_cached(v[0].x), as_cached(v[0].y));
         }
         sync();
 #pragma unroll
@@ -593,8 +592,8 @@ __device__ __forceinline__ void attention(const Step& st, uint32_t l) {
         const uint32_t t = base + u * (NW * PPW) + grp;
         if (base + u * (NW * PPW) >= t1) break;  // the whole warp
         float kf[8], vf[8];
-        KV8<KVT>::unpack(kr[u], kf);
-        KV8<KVT>::unpack(vr[u], vf);
+        KV8::unpack(kr[u], kf);
+        KV8::unpack(vr[u], vf);
         take(kf, vf, t < t1 && t != newest);
       }
       base += NW * PPW * UNR;
@@ -743,7 +742,7 @@ drain:  // nothing is on its way into this CTA's memory when it leaves, neither 
 }
 
 // ---- the step ----------------------------------------------------------------------------------------------------------------
-template <typename KVT, int D>
+template <int D>
 __global__ void __launch_bounds__(kAllThreads, 1) step_resident_kernel(const __grid_constant__ ResidentStep launch) {
   extern __shared__ __align__(1024) char smem[];
   Shared& sh = *reinterpret_cast<Shared*>(smem + kSharedOffset);
@@ -824,10 +823,10 @@ __global__ void __launch_bounds__(kAllThreads, 1) step_resident_kernel(const __g
     for (uint32_t k = 0; k < end; ++k) {
       const uint32_t l = k >> 2, ph = l < p.L ? k & 3u : (uint32_t)PH_HEAD;
       if (ph == PH_O) {
-        attention<KVT, D>(st, l);
+        attention<D>(st, l);
         sync();
       }
-      product<KVT, D>(st, xc, acc, l, ph);
+      product<D>(st, xc, acc, l, ph);
       sync();
     }
     if (warp == 0 && dead(sh) < 2)  // (the products' arrivals on the last pieces of x)
@@ -891,10 +890,7 @@ __global__ void __launch_bounds__(kAllThreads, 1) step_resident_kernel(const __g
 }
 
 using Kernel = void (*)(const ResidentStep);
-Kernel pick(int kvdtype, uint32_t d) {
-  if (kvdtype == 1) return d == 32 ? step_resident_kernel<__half, 32> : d == 64 ? step_resident_kernel<__half, 64> : step_resident_kernel<__half, 128>;
-  return d == 32 ? step_resident_kernel<float, 32> : d == 64 ? step_resident_kernel<float, 64> : step_resident_kernel<float, 128>;
-}
+Kernel pick(uint32_t d) { return d == 32 ? step_resident_kernel<32> : d == 64 ? step_resident_kernel<64> : step_resident_kernel<128>; }
 
 }  // namespace
 
@@ -914,7 +910,11 @@ size_t resident_words_per_layer(uint32_t H, uint32_t qH, uint32_t kvH, uint32_t 
 
 bool resident_plan(int wdtype, int kvdtype, ResidentStep* p) {
   const uint32_t qDim = p->qH * p->d, G = sm_count();
-  if (wdtype != 1) return false;
+  // Sums inside the tensor core lose more than sums in registers, the more the longer they are. A float16 cache rounds by a thousand times
+  // as much, and logits are off by the same either way; with a float32 cache they were off by more (1B architecture, two layers, position
+  // 0: 7.1e-7 for 4.8e-7 as launches, one layer's rows 8.5e-7 for 3.4e-7). Shorter sums, a 512-column piece each, are as exact as
+  // the launches and take what the one kernel gains (480 -> 546 us a step).
+  if (wdtype != 1 || kvdtype != 1) return false;
   if (p->d != 32 && p->d != 64 && p->d != 128) return false;
   if (p->H % 64 || qDim % 64 || p->F % 64) return false;  // rows of whole blocks of 64 columns
   if (p->H > kMaxNarrow || qDim > kMaxNarrow || p->F > kMaxWide) return false;
@@ -934,7 +934,7 @@ bool resident_plan(int wdtype, int kvdtype, ResidentStep* p) {
     for (int b = 0; b < 4; ++b)
       if (!encode_stack_map16(reinterpret_cast<CUtensorMap*>(p->maps[i][b]), p->w[i], rows[i], cols[i], i == PH_HEAD ? 1 : p->L, p->layer_stride, kTileRows >> b, kPiece / 64))
         return false;
-  const Kernel k = pick(kvdtype, p->d);
+  const Kernel k = pick(p->d);
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, (int)kAllThreads, kSmem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
@@ -943,8 +943,8 @@ bool resident_plan(int wdtype, int kvdtype, ResidentStep* p) {
   return true;
 }
 
-cudaError_t launch_step_resident(cudaStream_t s, int kvdtype, const ResidentStep& p) {
-  const Kernel k = pick(kvdtype, p.d);
+cudaError_t launch_step_resident(cudaStream_t s, const ResidentStep& p) {
+  const Kernel k = pick(p.d);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};

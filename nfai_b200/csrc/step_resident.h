@@ -8,7 +8,7 @@ struct ResidentArgs {
   const void* w[5] = {};              // QKV, O, gate/up and down of layer 0, the head
   const float *attn_norm = nullptr, *ffn_norm = nullptr;  // of layer 0
   uint64_t layer_stride = 0;          // bytes from a layer's weights and gains to the next one's
-  void *kc = nullptr, *vc = nullptr;  // [L][ctx][kvH*d]
+  void *kc = nullptr, *vc = nullptr;  // [L][ctx][kvH*d] float16
   uint32_t L = 0, H = 0, qH = 0, kvH = 0, d = 0, F = 0, V = 0, ctx = 0, ropeDim = 0;
   float eps = 0.f;
   const void* embd = nullptr;
@@ -39,6 +39,6 @@ size_t resident_words_per_layer(uint32_t H, uint32_t qH, uint32_t kvH, uint32_t 
 uint32_t resident_positions(uint32_t d);
 // Fills in the launch's layout; false where the sizes, types or the device do not fit (the step is then a sequence of launches).
 bool resident_plan(int wdtype, int kvdtype, ResidentStep* p);
-cudaError_t launch_step_resident(cudaStream_t s, int kvdtype, const ResidentStep& p);
+cudaError_t launch_step_resident(cudaStream_t s, const ResidentStep& p);
 
 }  // namespace nfai
