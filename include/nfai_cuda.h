@@ -290,7 +290,8 @@ int nfai_model_set_prefetch(nfai_model* m, uint64_t lookahead_bytes, uint64_t ex
 int nfai_step_launches(const nfai_model* m, int* out);
 
 /* Number of kernels that the step at the current position launches: 1 where the whole step is one resident kernel (float16
- * models of some size with a float16 cache of up to 4 096 positions on one GPU, no launch shapes or look-ahead asked for), else as above. */
+ * models of some size with a float16 cache of up to 4 096 positions on one GPU, no launch shapes or look-ahead asked for, and a
+ * position below a line that follows from the heads: 2 048 for 32 heads of 128, 3 072 for 24, 4 096 for 32 of 64), else as above. */
 int nfai_step_kernels(const nfai_model* m, int* out);
 
 /* ---- single kernels on caller-owned DEVICE buffers (kernel-level parity tests, embedding in other hosts) - */

@@ -415,7 +415,7 @@ void bind_resident(nfai_model* m, char* words, char* counts) {
 
 // Whether the step at position `pos` is one kernel: launch shapes and an L2 look-ahead belong to a sequence of launches.
 bool steps_resident(const nfai_model* m, uint32_t pos) {
-  return m->resident && !m->shaped && !m->pf_look && !m->pf_extra && pos < resident_positions(m->hp.d);
+  return m->resident && !m->shaped && !m->pf_look && !m->pf_extra && pos < resident_positions(m->step);
 }
 
 // The step at position `pos`: where the model stands when it runs.

@@ -33,6 +33,8 @@
 // 2 846 -> 2 746. Small layers have nothing to stream meanwhile: 13 MB a layer 43 -> 46, 5 MB 41 -> 43.
 #include <math.h>
 
+#include <algorithm>
+
 #include "attn_core.cuh"
 #include "common.cuh"
 #include "kernels.h"
@@ -894,10 +896,13 @@ Kernel pick(uint32_t d) { return d == 32 ? step_resident_kernel<32> : d == 64 ? 
 
 }  // namespace
 
-// Positions up to which this kernel's attention keeps the step ahead of the sequence of launches. It reads a KV head's rows once for
-// every query head, which heads of 128 feel first (3B: 1 682 -> 1 651 us a step at position 3 000, 1 721 -> 1 767 at 4 000; 8B
-// 3 151 -> 3 235 at 4 000; heads of 64, 1B: 733 -> 718 at 4 000).
-uint32_t resident_positions(uint32_t d) { return d == 128 ? 3072 : 4096; }
+// Positions up to which this kernel's attention keeps the step ahead of the sequence of launches. What grows with them is a CTA's
+// share of a head, position / splits rows of d keys and values, read while no product has its x: the line is at 65 536 elements of each.
+// us a step, launches and this kernel: 1B (32 heads of 64, 4 ranges: 4 096) at 4 070 666 and 651; 3B (24 of 128, 6 ranges: 3 072) at
+// 3 060 1 691 and 1 675, 3 400 1 713 and 1 706, 4 000 1 736 and 1 774; 8B (32 of 128, 4 ranges: 2 048) at 1 600 3 052 and 3 039,
+// 1 900 3 055 and 3 079, 3 060 3 150 and 3 217; 7B with as many KV heads at 2 300 2 883 and 2 873, 2 500 2 896 and 2 903; 8 layers
+// with 64 heads of 64 (2 ranges: 2 048), 8 KV heads: 2 800 728 and 719, 3 100 736 and 739, 64 KV heads: 1 300 786 and 776, 1 600 794 and 805.
+uint32_t resident_positions(const ResidentArgs& p) { return std::min(65536u * p.splits / p.d, 4096u); }
 
 uint32_t resident_splits(uint32_t qH) {
   const uint32_t s = sm_count() / qH;
@@ -918,7 +923,9 @@ bool resident_plan(int wdtype, int kvdtype, ResidentStep* p) {
   if (p->d != 32 && p->d != 64 && p->d != 128) return false;
   if (p->H % 64 || qDim % 64 || p->F % 64) return false;  // rows of whole blocks of 64 columns
   if (p->H > kMaxNarrow || qDim > kMaxNarrow || p->F > kMaxWide) return false;
-  // Weights of a layer that are worth it: 5 and 13 MB lose 2 us a step, 121 MB win 5.
+  // Weights of a layer that are worth it even if it is the only one and stays in L2: layers of 18 MB, position 128, launches and this
+  // kernel: one layer 24.8 and 28.9 us a step, two 43.2 and 45.3, four 82.2 and 73.9; of 39 MB: 32.9 and 33.0, 56.4 and 51.4; of 56
+  // MB: 35.1 and 35.9, 61.2 and 56.1; of 116 MB: 45.1 and 43.9, 78.1 and 71.8.
   if (((uint64_t)p->H * (2 * qDim + 2 * p->kvH * p->d) + (uint64_t)3 * p->H * p->F) * 2 < (32u << 20)) return false;
   if (p->H / 2 / G + 1 > 32) return false;                // the kept residual; rows of down are one block
   if (p->H / 2 < G || (p->qH + 2 * p->kvH) * p->d / 2 < G || p->F < G || p->V < G) return false;  // no CTA without a row

@@ -35,8 +35,8 @@ struct ResidentStep : ResidentArgs {
 };
 
 size_t resident_words_per_layer(uint32_t H, uint32_t qH, uint32_t kvH, uint32_t d, uint32_t F);
-// Steps from this position on are a sequence of launches.
-uint32_t resident_positions(uint32_t d);
+// Steps from this position on are a sequence of launches (p as resident_plan left it).
+uint32_t resident_positions(const ResidentArgs& p);
 // Fills in the launch's layout; false where the sizes, types or the device do not fit (the step is then a sequence of launches).
 bool resident_plan(int wdtype, int kvdtype, ResidentStep* p);
 cudaError_t launch_step_resident(cudaStream_t s, const ResidentStep& p);

@@ -184,3 +184,30 @@ def test_a_look_ahead_runs_the_launches_it_belongs_to(factory, monkeypatch):
         m.set_prefetch(0)
         assert m.step_kernels() == 1
         m.Dispose()
+
+
+@pytest.mark.parametrize("qH,kvH,d", [(32, 8, 64), (24, 8, 128), (32, 8, 128), (64, 8, 64), (64, 16, 32)])
+def test_which_step_runs(factory, qH, kvH, d):
+    """On either side of the line, where a CTA's share of a head is 65 536 elements: the one kernel and the launches agree to what a
+    float16 row that goes either way makes of float32 sums in another order."""
+    cfg = synth.get_config("s1", V=2053, qH=qH, kvH=kvH, d=d)
+    splits = min(16, torch.cuda.get_device_properties(0).multi_processor_count // qH)
+    line = min(65536 * splits // d, 4096)
+    rng = np.random.default_rng(line)
+    rows = [[rng.standard_normal((line, cfg.kvDim)).astype(np.float32) for _ in "kv"] for _ in range(cfg.L)]
+    got = []
+    for shaped in (False, True):
+        m = create_synthetic_model(cfg, 4096, factory=factory, kv_dtype="f16")
+        if shaped:
+            m.tune("ffn_gate_up", 0, 2, 4, 2)
+        for position in (line - 1, line):
+            if position < 4096:
+                for l in range(cfg.L):
+                    m.write_kv_range(l, 0, *rows[l])
+                m.set_position(position)
+                assert (m.step_kernels() == 1) == (not shaped and position < line)
+                got.append(m.decode(3)[0])
+        m.Dispose()
+    n = len(got) // 2
+    assert all(off(a, torch.from_numpy(b)) < 1e-4 for a, b in zip(got[:n], got[n:]))
+    assert n == 1 or np.array_equal(got[1], got[3])
