@@ -244,6 +244,8 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_prefill_umma_kernel(const __g
           if (it) {
             Values::at_rescaling(it, value);
             fence_after();
+            // a row that has seen no position yet: what zero weights left of values that are not finite goes, as if it had begun here
+            const bool begins = m == kNegBig;
             const float f = gqa_ex2(m - top);
             l *= f;
 #pragma unroll 1
@@ -251,7 +253,7 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_prefill_umma_kernel(const __g
               uint32_t o[16];
               tmem_ld(lanes + kO + c, o);
 #pragma unroll
-              for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
+              for (int e = 0; e < 16; ++e) o[e] = begins ? 0u : __float_as_uint(__uint_as_float(o[e]) * f);
               tmem_st(lanes + kO + c, o);
             }
           }

@@ -192,6 +192,26 @@ def test_prompt_attention_on_whole_tiles(cuda_ctx, mixer, portions, monkeypatch)
     assert U.error(got["1"], got["2"]) < 8 * 2.0 ** -9
 
 
+@pytest.mark.parametrize("dim", [64, 128])
+def test_a_row_that_is_not_a_number(cuda_ctx, dim, monkeypatch):
+    """A token whose embedding is infinite has queries, keys and values that are not numbers: neither are it and the rows that see it, and
+    rows before its tile of keys (64 positions) are untouched, in the tensor-core and in the warp-level kernel."""
+    cfg = U.config([U.layer(U.attn(8, 2, dim, dim, scale=51.2 / dim))], 64, 96)
+    W = U.weights(cfg, 13)
+    W["embed"][95] = np.inf
+    m = build(cuda_ctx, cfg, W, "bf16", 256)
+    toks = np.random.default_rng(dim).integers(0, 95, 200).tolist()
+    for kind in ("1", "2"):
+        monkeypatch.setenv("NFAI_PREFILL_ATTN", kind)
+        rows = []
+        for token in (95, 94):
+            m.reset()
+            rows.append(m.forward(toks[:100] + [token] + toks[101:], range(200)))
+        assert np.isfinite(rows[1]).all()
+        assert np.isnan(rows[0][100:]).all() and np.array_equal(rows[0][:64], rows[1][:64]), kind
+    m.Dispose()
+
+
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 def test_feed_forward_alone(cuda_ctx, dtype):
     """The attention's output matrix is zero (its bias stays): what is left are clamped feed-forwards and the residual. Values
