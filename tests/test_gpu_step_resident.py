@@ -1,4 +1,6 @@
 """The decode step as one resident kernel, against a plain float64 statement and against the same step as a sequence of launches."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -211,3 +213,40 @@ def test_which_step_runs(factory, qH, kvH, d):
     n = len(got) // 2
     assert all(off(a, torch.from_numpy(b)) < 1e-4 for a, b in zip(got[:n], got[n:]))
     assert n == 1 or np.array_equal(got[1], got[3])
+
+
+def test_steps_and_prompts_of_two_threads(factory):
+    """Two contexts on one GPU, a thread each: every step of one needs all of the GPU's SMs at once, whatever the other has running
+    there, and waits for them; results are those of either alone."""
+    cfg = synth.get_config("s1", V=2053)
+    other = LlamaModelFactory(0)
+    models = [create_synthetic_model(cfg, 512, factory=f) for f in (factory, other)]
+    prompts = [synth.prompt_ids(cfg, n, 4) for n in (5, 160)]
+
+    def work(m, ids, rounds):
+        out = []
+        for _ in range(rounds):
+            m.reset()
+            _, best = m.prefill(ids)
+            answer, _ = m.decode_greedy(best, 60)
+            out.append([list(answer)] + [m.decode(int(t))[0].tolist() for t in ids[:5]])
+        return out
+
+    want = [work(m, ids, 1)[0] for m, ids in zip(models, prompts)]
+    got, failed = [None, None], []
+
+    def run(i):
+        try:
+            got[i] = work(models[i], prompts[i], 6)
+        except Exception as e:  # noqa: BLE001
+            failed.append(e)
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(120)
+    assert not failed and all(g == [w] * 6 for g, w in zip(got, want))
+    for m in models:
+        m.Dispose()
+    other.Dispose()
