@@ -67,23 +67,6 @@ __device__ __forceinline__ uint32_t u_half2(float a, float b) {
   __half2 h = __floats2half2_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
 }
-// Two float32 operations per instruction
-__device__ __forceinline__ uint64_t pair(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpair(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 // 2^x of a pair on the fused multiply-add units, for x below 128: x = n + f with n whole and |f| <= 1/2 (adding 1.5 * 2^23 rounds),
 // 2^f by its minimax polynomial of degree 5 (a linear program over the relative error; 2.1e-7 in float32, as much as the
 // hardware's approximation is allowed), n added to the exponent. Anything below 2^-126 becomes that; a NaN becomes the largest

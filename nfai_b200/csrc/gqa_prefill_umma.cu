@@ -43,23 +43,6 @@ struct Smem {
   static constexpr uint32_t kTotal = kSwapOff + 2 * kM * 4 + 1024;
 };
 
-// Two float32 operations per instruction
-__device__ __forceinline__ uint64_t pair(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpair(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 __device__ __forceinline__ uint32_t bf2(float a, float b) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return reinterpret_cast<const uint32_t&>(h);
