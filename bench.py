@@ -2,7 +2,7 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--config c1]
 
-A step is one decoded token (one replay of the captured decode step). At N = 1 the workload is the
+A step is one decoded token. At N = 1 the workload is the
 Llama-3.2-1B-architecture FP16 model, 128-token random prompt, then K greedy decode steps; for N > 1 the same
 model runs tensor-parallel over the N GPUs (strong scaling), one rank per GPU under torchrun.
 Prints ONE JSON line on rank 0.
@@ -11,8 +11,10 @@ Prints ONE JSON line on rank 0.
              on the library's stream, max over ranks.
   e2e        tokens/s through the reference-facing call (nfai_decode): host token in, arg-max out, copies and
              synchronisation inside the timed region.
-  roofline   the dominant kernel (FFN gate/up GEMV): algorithmic bytes per launch / mean launch time, against the
-             measured HBM copy bandwidth.
+  roofline   the dominant kernel: algorithmic bytes per launch / mean launch time, against the measured HBM copy bandwidth.
+             Where the step is one kernel, that kernel inside the timed loop; else the FFN gate/up GEMV, timed alone.
+  kernels    the launches of a step that is a sequence of them, each timed alone (one GPU steps of float16 models with short
+             caches are one kernel and launch none of these).
   cpu_baseline  the CPU oracle (a port of the reference's arithmetic; the reference itself needs .NET + Vulkan and
              cannot run here) timed on the host cores on a few tokens of the same workload.
 
@@ -36,13 +38,12 @@ if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
 FALLBACK_HBM_GBS = 6650.0
-# dram__bytes_read.sum + dram__bytes_write.sum of one launch of the dominant kernel (FFN gate/up GEMV of configs[1]
-# on one GPU), from an ncu capture of this kernel; it goes stale when the kernel's memory behaviour changes, so the
-# capture it came from is named beside it.
-NCU_TRAFFIC = {("c1", 1): {"bytes": 67165440 + 710400,
-                           "capture": "ncu --set full --clock-control none -k regex:gemv_kernel -s 170 -c 4 of "
-                                      "bench.py --steps 2 --warmup 3 --prompt-len 2 --min-timed-s 0: the gate/up launch "
-                                      "(67.165 MB read + 0.710 MB written against 67.117 MB algorithmic)"}}
+# dram__bytes_read.sum + dram__bytes_write.sum of one launch of the dominant kernel, from an ncu capture of that kernel; it goes
+# stale when the kernel's memory behaviour changes, so the capture it came from is named beside it.
+NCU_TRAFFIC = {("c1", 1): {"bytes": 2473121024 + 4728576,
+                           "capture": "ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k regex:step_resident "
+                                      "-s 6 -c 2 of bench.py --steps 2 --warmup 3 --prompt-len 2 --min-timed-s 0: one step at a position "
+                                      "below 8 (2473.1 MB read + 4.7 MB written against 2471.9 MB algorithmic)"}}
 PROMPT_LEN = 128
 MIN_TIMED_S = 1.0  # the K-step loop is repeated until this much device time has been measured; the median is reported
 
@@ -308,7 +309,13 @@ def run_ours(args, cfg):
     clocks = sampler.stop() if rank == 0 else None
     same_tokens = [int(t) for t in toks] == [int(t) for t in e2e_toks]
 
-    # ---- roofline of the dominant kernel, timed alone with events on the same stream
+    # ---- which kernels the timed steps were
+    step_kernels = []
+    for p in range(PROMPT_LEN + W, PROMPT_LEN + W + K):
+        model.set_position(p)
+        step_kernels.append(model.step_kernels())
+    one_kernel = max(step_kernels) == 1
+    # ---- the launches of a step, timed alone with events on the same stream
     peak, peak_kind = measured_peak()
     kern = {}
     for name in ("ffn_gate_up", "ffn_down", "qkv_rope", "attn_out", "lm_head", "attention"):
@@ -349,7 +356,6 @@ def run_ours(args, cfg):
                   "frac_of_sustained_bf16": flops / tsec / 1e12 / sus, "frac_of_burst_bf16": flops / tsec / 1e12 / burst,
                   "peak_kind": kind, "timing": "host clock around nfai_prefill with a synchronise on both sides, median of 5",
                   "flops": "2 x layer matrix params x T + causal attention 2 T^2 qDim L + one LM-head row"}
-    launches = model.step_kernels()
     kv_bytes = 2 if model.kv_dtype == "f16" else 4
     first_pos = PROMPT_LEN + W
     step_bytes = sum(synth.decode_bytes(cfg, p, kv_bytes) for p in range(first_pos, first_pos + K)) / K / world
@@ -361,7 +367,12 @@ def run_ours(args, cfg):
             dist.destroy_process_group()
         return
 
-    dom = kern["ffn_gate_up"]
+    if one_kernel:
+        dom = {"kernel": "step_resident_kernel (a whole decode step)", "us": ms / K * 1e3, "bytes": step_bytes,
+               "gbs": step_bytes / (ms / K * 1e-3) / 1e9}
+    else:
+        dom = dict(kern["ffn_gate_up"], kernel="gemv_kernel (FFN gate/up + RMSNorm + SiLU*up)")
+    traffic = NCU_TRAFFIC.get((args.config, world)) if one_kernel else None
     value = K / (ms * 1e-3)
     line = {
         "metric": "decode tok/s (batch 1)", "value": value, "unit": "tok/s", "n_gpus": world, "steps": K, "warmup": W,
@@ -376,10 +387,10 @@ def run_ours(args, cfg):
                    "seed": args.seed},
         "e2e": {"value": K / e2e_s, "unit": "tok/s", "h2d_bytes_per_step": 4, "d2h_bytes_per_step": 32,
                 "same_tokens_as_device_loop": same_tokens},
-        "gpu_launches": K * launches,
-        "roofline": {"bound": "hbm", "kernel": "gemv_kernel (FFN gate/up + RMSNorm + SiLU*up)", "achieved": dom["gbs"],
-                     "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": dom["gbs"] / peak, "traffic": (NCU_TRAFFIC.get((args.config, world)) or {}).get("bytes"),
-                     "traffic_capture": (NCU_TRAFFIC.get((args.config, world)) or {}).get("capture"),
+        "gpu_launches": sum(step_kernels),
+        "roofline": {"bound": "hbm", "kernel": dom["kernel"], "achieved": dom["gbs"],
+                     "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": dom["gbs"] / peak,
+                     "traffic": (traffic or {}).get("bytes"), "traffic_capture": (traffic or {}).get("capture"),
                      "launch_us": dom["us"], "bytes_per_launch": dom["bytes"]},
         "step_roofline": {"bytes_per_token_per_gpu": step_bytes, "achieved_gbs": step_bytes / (ms / K * 1e-3) / 1e9,
                           "frac_of_8tbs": step_bytes / (ms / K * 1e-3) / 8e12,
@@ -552,7 +563,7 @@ def run_design(args):
         snap.close()
         pf, step = statistics.median(times), statistics.median(ms)
         return {"prefill_tokens": T, "prefill_ms": pf * 1e3, "prefill_tok_s": T / pf, "decode_ms": step, "decode_tok_s": 1e3 / step,
-                "decode_e2e_tok_s": 1 / e2e, "launches_per_step": model.step_launches(), "kernels": kern}
+                "decode_e2e_tok_s": 1 / e2e, "launches_per_step": model.step_kernels(), "kernels": kern}
 
     def rates(r, params, z):
         r["layer_matrix_params"] = params
