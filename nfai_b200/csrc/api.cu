@@ -370,8 +370,8 @@ int capture(nfai_model* m, bool with_head, bool from_prompt, cudaGraphExec_t* ou
   return NFAI_OK;
 }
 
-// Whether the step can run as one resident kernel, and its layout. One GPU, caches of up to 4 096 positions (beyond, attention is most
-// of the step and runs on the tensor cores).
+// Whether the step can run as one resident kernel, and its layout. One GPU, caches of up to 4 096 positions: models with larger ones
+// share a pass over the cache among query heads (attn_heads), which this kernel does not, and keep the launches at every position.
 bool plan_resident(nfai_model* m) {
   nfai_ctx* c = m->ctx;
   const nfai_hparams& hp = m->hp;

@@ -11,8 +11,9 @@
 // there when this one's weights are done, and two CTAs share an SM. A row's sums are rescaled only when its maximum has grown by more
 // than 8 (base 2): weights are then at most 2^8 and their relative rounding is what it was.
 //
-// What bounds it: issue slots of the softmax (bias, exponential, split: about 11 per pair of weights). Against the warp-level kernel of
-// gqa_prefill.cu, prompts of 16 layers with 32 heads of 64 (ms): 2011 tokens 6.54 and 5.97 (about 75 and 39 us a layer), 1024: 4.00 and
+// What bounds it: issue slots of the softmax (bias, exponential, split: about 11 per pair of weights) are 53 % of a launch's, the rest is
+// latency between a tile's steps and the last of 1.7 waves (41 us at 2011 tokens). Against the warp-level kernel of
+// gqa_prefill.cu, prompts of 16 layers with 32 heads of 64 (ms): 2011 tokens 6.52 and 5.99 (about 75 and 41 us a layer), 1024: 4.00 and
 // 3.91, 512: 3.04 and 2.99, 384: 2.88 and 2.83. Tiles of 128 positions, their weights over the scores of the only tile that fits beside
 // O then: 6.18 at 2011 (spills, and the products wait for the weights and the weights for the products).
 #include "attn_phases.h"

@@ -9,8 +9,8 @@
 // ahead of the products while those wait for x.
 //
 // For that to help, the ring must be emptied much faster than HBM fills it (23 bytes per clock and SM). With float32 arithmetic on
-// the warps it was not: 25 bytes, half of the instructions conversions and sums across lanes, 549 us a step of the 1B architecture;
-// with warp-level products 39 bytes and 548 us. So tcgen05 multiplies, exactly: float16 weights are the A operand as they lie in the
+// the warps it was not: 25 bytes, half of the instructions conversions and sums across lanes, and little more with warp-level products (39
+// bytes). So tcgen05 multiplies, exactly: float16 weights are the A operand as they lie in the
 // ring, x is split into three float16 terms of 11 bits each, scaled to the largest element of its block, as the B operand. Every
 // product is exact and sums are float32 in tensor memory (resident_plan says what they lose); one thread issues them, and no warp
 // touches a weight.
@@ -28,9 +28,10 @@
 // range of positions; the rows of earlier positions are requested before the new row's words are polled; ranges are merged by the
 // CTAs that made them, a slice each.
 //
-// Measured (B200, us a step at position 128, sequence of launches -> this kernel; layer weights per step in brackets): 1B architecture
-// (121 MB a layer) 605 -> 529, at position 700 673 -> 553, at 4 000 733 -> 718; 3B 1 487 -> 1 321, at 4 000 1 721 -> 1 767; 8B
-// 2 846 -> 2 746. Small layers have nothing to stream meanwhile: 13 MB a layer 43 -> 46, 5 MB 41 -> 43.
+// Measured (B200, us a step, sequence of launches -> this kernel): 1B architecture (121 MB a layer) at position 128 619 -> 535, 391 629
+// -> 550, 700 675 -> 558, 2 000 691 -> 629, 4 000 734 -> 725; 3B at 128 1 477 -> 1 332, 1 000 1 672 -> 1 485; 8B at 128 2 886 -> 2 747,
+// 1 000 3 036 -> 2 948. What single choices are worth, below, is at position 128 of the 1B architecture with a head of 32 768 rows (478 to
+// 481 from one board to the next).
 #include <math.h>
 
 #include <algorithm>
@@ -77,9 +78,9 @@ __device__ __forceinline__ void copy_box(unsigned long long policy, uint32_t dst
       "l"(map), "r"(0), "r"(row), "r"(block), "r"(layer), "r"(bar), "l"(policy)
       : "memory");
 }
-// The thread's number, asked for where it is used: what the compiler would otherwise derive from it once and keep over all phases
-// of all layers ends up in local memory, which here means L2: next to the ring there is no L1 to speak of. (With 180 bytes of
-// it a thread a step of the 1B architecture took 724 us.)
+// The thread's number, asked for where it is used: the compiler would otherwise derive things from it once and keep them over all phases
+// of all layers (168 registers a thread, 144 so; beyond 200 they would go to local memory, which here means L2: next to the ring
+// there is no L1 to speak of).
 __device__ __forceinline__ uint32_t thread_id() {
   uint32_t t;
   asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
@@ -143,6 +144,7 @@ __device__ __forceinline__ void give_up(Shared& sh, StepState* state, uint32_t h
   atomicMax(&sh.dead, how);
   atomicOr(&state->err, 4u);
 }
+// (inlined: 481.1 us a step, 484.7 as a function of its own)
 __device__ __forceinline__ void wait_slowly(Shared& sh, StepState* state, uint32_t bar, uint32_t parity, unsigned long long limit) {
   const unsigned long long t0 = global_timer_ns();
   for (uint32_t polls = 1; !bar_try(bar, parity) && dead(sh) < 2; ++polls)
@@ -276,7 +278,7 @@ __device__ __forceinline__ void issue_products(const Step& st) {
         st.wait(sh.acc_empty[acc.slot], acc.turn ^ 1u);
 #pragma unroll 1
         for (uint32_t i = 0; i < n; ++i, w.next(kSlots), x.next(kXSlots)) {
-          // (one decision a piece: with votes behind the other two waits as well the 1B architecture took 486.6 us a step, 481.5 so)
+          // (one decision a piece: with votes behind the other two waits as well 486.6 us a step, 481.5 so)
           if (r == 0) st.wait(sh.x_full[x.slot], x.turn);
           if (!st.warp_wait(sh.full[w.slot], w.turn)) return;
           umma::fence_after();
@@ -410,7 +412,7 @@ __device__ __forceinline__ void put_x(const Step& st, Cursor& xc, uint32_t t, ui
     st.wait(sh.x_empty[xc.slot], xc.turn ^ 1u);
 #pragma unroll
     for (uint32_t i = 0; i < 3; ++i) sts4(x_row(st.xs + xc.slot * kXBytes, block, i, lane), term[i]);
-    // (a fence a piece: the products begin with the first while the others are made; one for all 533 -> 559 us a step)
+    // (a fence a piece: the products begin with the first while the others are made; one for all of a chunk 502.0 us a step, 477.8 so)
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if (lane == 0) bar_arrive(s_addr(&sh.x_full[xc.slot]));
@@ -687,13 +689,14 @@ __device__ __forceinline__ void attention(const Step& st, uint32_t l) {
 // ---- the weights' way into the ring -----------------------------------------------------------------------------------------
 // A warp copies this CTA's shares in the order they are used: tile by tile, 512 columns at a time. A slot's copies are begun when it
 // is free and the ones kAhead before them have landed: what is in flight keeps HBM busy and no more, because everything else that
-// misses L2 (words that were written, gains, K and V) queues behind it. (The whole ring in flight is 4 us of HBM time: 842 us a step
-// against 724.) The last rows of a share come in boxes of 8, 4 and 2, so that no row is read that is another CTA's. (One copy per row
-// instead, 1 KB each, took 119 us a step of two layers against 78: they are issued one by one.)
+// misses L2 (words that were written, gains, K and V) queues behind it. (The whole ring in flight is 4 us of HBM time; it made no
+// difference at short positions, 480.0 us a step and 481.1.) The last rows of a share come in boxes of 8, 4 and 2, so that no row is read
+// that is another CTA's. (One copy per row instead, 1 KB each, took a step of two layers half as long again: they are issued one by
+// one.) The warp's waits are votes: its lanes on their own ahead of one vote took 484.8 us a step, 478.7 so.
 __device__ __forceinline__ void feed(const Step& st, const ResidentStep& launch) {
   const ResidentArgs& p = st.sh.p;
   Shared& sh = st.sh;
-  unsigned long long once;       // weights are read once a step: they give way to everything else in L2 (564 us a step without, 550 with)
+  unsigned long long once;       // weights are read once a step: they give way to everything else in L2 (502.3 us a step without, 481.1 with)
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once));
   Cursor c, landed;
   uint32_t begun = 0, seen = 0;  // copies, and those that were waited for
